@@ -216,166 +216,396 @@ __global__ void beam_dense_kernel(int64_t n_nodes, const int32_t* __restrict__ r
 }
 
 // Blocked right-looking LU with partial pivoting and the solve of A x = b (x overwrites b),
-// in panels of kLuPanel columns: per panel
-//   beam_lu_panel_kernel   (one CTA)   pivots, row swaps, multipliers and rank-1 updates inside
-//                                      the panel's columns, and the forward elimination of b;
-//   beam_lu_swap_trsm_kernel (a thread per trailing column) the panel's row swaps and
-//                                      U12 = L11^-1 A12 on the columns right of the panel;
-//   beam_lu_update_kernel  (32 x 32 tiles) A22 -= L21 U12, each element subtracting the
-//                                      panel's terms in column order;
-// then beam_lu_backsub_kernel (one CTA).  Every element sees the unblocked algorithm's
-// operations in its order (fused multiply-adds), so the factors and x do not depend on the
-// panel width.  The multipliers of earlier panels are never read again (b is eliminated as
-// the panels go), so row swaps touch the panel, the trailing columns and b only.
+// in panels of NB columns, limited to the band of the matrix: with half bandwidth kb (the largest
+// |i - j| of a nonzero) column k of the factors ends at row k + kb and, with row exchanges, row k
+// at column k + 2 kb; outside, every operation of the dense algorithm has a zero operand and
+// changes nothing.  Per panel
+//   beam_lu_panel_kernel    (one CTA)   pivots, row swaps, multipliers and rank-1 updates inside
+//                                       the panel's columns, and the forward elimination of b;
+//   beam_lu_trailing_kernel (a CTA per 32 trailing columns) the panel's row swaps, then
+//                                       U12 = L11^-1 A12, and with few rows below the panel also
+//                                       A22 -= L21 U12;
+//   beam_lu_update_kernel   (32 x 32 tiles) A22 -= L21 U12 where the rows are many;
+// then beam_lu_backsub_kernel (one CTA).  Every element sees the unblocked dense algorithm's
+// operations in its order (fused multiply-adds), so the factors and x depend neither on the panel
+// width nor on the band.  The multipliers of earlier panels are never read again (b is
+// eliminated as the panels go), so row swaps touch the panel, the trailing columns and b only.
 // status: 0 ok, 1 singular (a zero pivot column; the later kernels then see status != 0 and
 // return).  Every loop is bounded by n.
-constexpr int kLuPanel = 32;
+//
+// What bounds it: the serial chain of pivots.  A panel's rows stay in the registers of one CTA
+// (RPT rows of NB columns per thread), so a column costs two barriers, two three-step warp
+// reductions, a division and its multiply-adds instead of several passes over global memory;
+// NB x RPT is chosen so that the rows that the band leaves fit (dense_lu).  Measured on the
+// 10 x 10 frame (600 DOFs, kb = 65) against the same algorithm over all n rows and columns from
+// global memory: panel 165 -> 28 us, trailing columns 56 -> 11 us per panel, back substitution
+// 300 -> 48 us per solve, bit for bit the same x; ten load steps 95.7 -> 21.8 ms.
+constexpr int kLuThreads = 512;   // most threads of a panel
+constexpr int kLuMaxPanel = 32;   // widest panel
+constexpr int kLuFuseRows = 256;  // up to so many rows below the panel are updated by the trailing kernel
 
-__global__ void __launch_bounds__(1024) beam_lu_panel_kernel(int n, int k0, double* __restrict__ A,
-                                                             double* __restrict__ b, int* __restrict__ piv,
-                                                             int* __restrict__ status) {
-  __shared__ double sv[32];
-  __shared__ int si[32];
-  __shared__ int s_piv;
-  __shared__ double s_pv;
+// the panel's row exchanges, as one permutation: src[k] = the row that moves to panel row k; moved
+// pairs (dest, src) for the rows below the panel
+struct LuSwaps {
+  int src[kLuMaxPanel];
+  int n_moved;
+  int dest[kLuMaxPanel];
+  int from[kLuMaxPanel];
+};
+
+// argmax of (key, pos), ties to the smaller pos, over a warp; all lanes get the result.  One lane
+// usually has the largest high word alone.
+__device__ __forceinline__ void lu_warp_argmax(unsigned long long& key, int& pos, int& winner) {
+  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  unsigned best = __ballot_sync(0xffffffffu, hi == mh);
+  if (best & (best - 1)) {
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    const bool top = hi == mh && lo == ml;
+    const unsigned mp = __reduce_min_sync(0xffffffffu, top ? (unsigned)pos : 0x7fffffffu);
+    best = __ballot_sync(0xffffffffu, top && (unsigned)pos == mp);
+  }
+  winner = __ffs(best) - 1;
+  key = __shfl_sync(0xffffffffu, key, winner);
+  pos = __shfl_sync(0xffffffffu, pos, winner);
+}
+
+// rows k0 .. rend - 1 (at most RPT * blockDim), columns k0 .. k0 + NB - 1.
+//   * A row stays with its thread; an exchange changes only the positions that the two threads
+//     hold (moving the rows cost 600 of 2,100 cycles per column).
+//   * Every warp publishes its best candidate's row before the column's one barrier; after it,
+//     all threads pick the pivot among the warps' and read its row.
+//   * The rows rotate by one column per step -- the current column is always a[.][0], a finished
+//     one (a multiplier below the pivot, an entry of U above) goes to the end -- so the loop over
+//     the columns stays rolled.
+template <int NB, int RPT>
+__global__ void __launch_bounds__(kLuThreads) beam_lu_panel_kernel(int n, int k0, int rend, double* __restrict__ A,
+                                                                   double* __restrict__ b,
+                                                                   LuSwaps* __restrict__ swaps,
+                                                                   int* __restrict__ status) {
+  constexpr int kWarps = kLuThreads / 32;
+  // per warp, in turns: its best candidate (zeros for the finished columns), the row's b, |value|
+  // as bits (ordered as |value| is; 0 also for NaN) and position
+  __shared__ __align__(16) double s_u[2][kWarps][NB];
+  __shared__ double s_rhs[2][kWarps];
+  __shared__ unsigned long long s_key[2][kWarps];
+  __shared__ int s_pos[2][kWarps];
+  __shared__ int s_moved;
   if (status[0] != 0) return;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  const int k1 = min(n, k0 + kLuPanel);
-  for (int k = k0; k < k1; ++k) {
-    // pivot: argmax |A[i][k]|, i >= k (ties -> smallest i)
-    double best = -1.0;
-    int bi = k;
-    for (int i = k + tid; i < n; i += nt) {
-      const double v = fabs(A[(int64_t)i * n + k]);
-      if (v > best) {
-        best = v;
-        bi = i;
-      }
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int m = rend - k0, w = min(NB, n - k0);
+  double a[RPT][NB], rhs[RPT];
+  int pos[RPT];  // the row's position in the exchanged order
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = tid + q * nt;
+    pos[q] = r;
+    rhs[q] = r < m ? b[k0 + r] : 0.0;
+    // n, k0 and w are even: 16-byte loads
+    const double2* __restrict__ row = reinterpret_cast<const double2*>(A + (int64_t)(k0 + (r < m ? r : 0)) * n + k0);
+#pragma unroll
+    for (int j = 0; j < NB; j += 2) {
+      const double2 v = (r < m && j < w) ? row[j / 2] : make_double2(0.0, 0.0);
+      a[q][j] = v.x;
+      a[q][j + 1] = v.y;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_down_sync(0xffffffffu, best, o);
-      const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) {
-        best = ov;
-        bi = oi;
-      }
-    }
-    if (lane == 0) {
-      sv[warp] = best;
-      si[warp] = bi;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      double bb = sv[0];
-      int ii = si[0];
-      for (int w = 1; w < nw; ++w)
-        if (sv[w] > bb || (sv[w] == bb && si[w] < ii)) {
-          bb = sv[w];
-          ii = si[w];
+  }
+  if (tid == 0) s_moved = 0;
+#pragma unroll 1
+  for (int c = 0; c < NB; ++c) {
+    const bool live = c < w;  // the ragged last panel only rotates its missing columns
+    const int t = c & 1;
+    int slot = 0;
+    if (live) {
+      unsigned long long key = 0;
+      int p = 0x7fffffff, mine = 0;
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        const double v = fabs(a[q][0]);
+        const unsigned long long kq =
+            (pos[q] >= c && pos[q] < m && v == v) ? (unsigned long long)__double_as_longlong(v) : 0;
+        if (kq > key || (kq == key && kq != 0 && pos[q] < p)) {
+          key = kq;
+          p = pos[q];
+          mine = q;
         }
-      s_piv = ii;
-      s_pv = bb;
-      piv[k - k0] = ii;
-      if (!(bb > 0.0)) status[0] = 1;
-    }
-    __syncthreads();
-    if (!(s_pv > 0.0)) return;
-    const int p = s_piv;
-    if (p != k) {  // the panel's columns and b
-      for (int j = k0 + tid; j < k1; j += nt) {
-        const double t = A[(int64_t)k * n + j];
-        A[(int64_t)k * n + j] = A[(int64_t)p * n + j];
-        A[(int64_t)p * n + j] = t;
       }
-      if (tid == 0) {
-        const double t = b[k];
-        b[k] = b[p];
-        b[p] = t;
+      int winner;
+      lu_warp_argmax(key, p, winner);
+      if (lane == winner) {
+        s_key[t][warp] = key;
+        s_pos[t][warp] = p;
+#pragma unroll
+        for (int q = 0; q < RPT; ++q)
+          if (q == mine) {
+#pragma unroll
+            for (int j = 0; j < NB; j += 2)
+              *reinterpret_cast<double2*>(&s_u[t][warp][j]) =
+                  make_double2(j < NB - c ? a[q][j] : 0.0, j + 1 < NB - c ? a[q][j + 1] : 0.0);
+            s_rhs[t][warp] = rhs[q];
+          }
+      }
+      __syncthreads();
+      key = lane < nw ? s_key[t][lane] : 0;
+      p = lane < nw ? s_pos[t][lane] : 0x7fffffff;
+      lu_warp_argmax(key, p, slot);
+      if (key == 0) {  // no pivot: uniform over the CTA
+        if (tid == 0) status[0] = 1;
+        return;
+      }
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        if (pos[q] == p)
+          pos[q] = c;
+        else if (pos[q] == c)
+          pos[q] = p;
       }
     }
-    __syncthreads();
-    const double pv = A[(int64_t)k * n + k];
-    for (int i = k + 1 + tid; i < n; i += nt) {
-      const double l = A[(int64_t)i * n + k] / pv;
-      A[(int64_t)i * n + k] = l;
-      b[i] = fma(-l, b[k], b[i]);
+    const double* __restrict__ su = s_u[t][slot];
+    const double pv = su[0], pr = s_rhs[t][slot];
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      double l = 0.0, last = a[q][0];
+      const bool below = live && pos[q] > c && pos[q] < m;
+      if (below && last != 0.0) {  // zeros (outside the band) would take the slow path of the division
+        l = last / pv;
+        rhs[q] = fma(-l, pr, rhs[q]);
+      }
+      if (below) last = l;
+      // one-column shift with the update; finished columns meet a zero
+      if (l != 0.0) {
+        a[q][0] = fma(-l, su[1], a[q][1]);
+#pragma unroll
+        for (int j = 2; j < NB; j += 2) {
+          const double2 v = *reinterpret_cast<const double2*>(su + j);
+          a[q][j - 1] = fma(-l, v.x, a[q][j]);
+          a[q][j] = fma(-l, v.y, a[q][j + 1]);
+        }
+      } else {
+#pragma unroll
+        for (int j = 1; j < NB; ++j) a[q][j - 1] = a[q][j];
+      }
+      a[q][NB - 1] = last;
     }
-    __syncthreads();
-    // rank-1 update of the panel's remaining columns: a warp per row
-    const double* __restrict__ pk = A + (int64_t)k * n;
-    for (int i = k + 1 + warp; i < n; i += nw) {
-      double* __restrict__ ai = A + (int64_t)i * n;
-      const double l = ai[k];
-      for (int j = k + 1 + lane; j < k1; j += 32) ai[j] = fma(-l, pk[j], ai[j]);
+  }
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = tid + q * nt;
+    if (r < m) {
+      double2* __restrict__ row = reinterpret_cast<double2*>(A + (int64_t)(k0 + pos[q]) * n + k0);
+#pragma unroll
+      for (int j = 0; j < NB; j += 2)
+        if (j < w) row[j / 2] = make_double2(a[q][j], a[q][j + 1]);
+      b[k0 + pos[q]] = rhs[q];
+      if (pos[q] < w) {
+        swaps->src[pos[q]] = k0 + r;
+      } else if (pos[q] != r) {  // at most one row per exchange: w of them
+        const int e = atomicAdd(&s_moved, 1);
+        swaps->dest[e] = k0 + pos[q];
+        swaps->from[e] = k0 + r;
+      }
     }
-    __syncthreads();
+  }
+  __syncthreads();
+  if (tid == 0) swaps->n_moved = s_moved;
+}
+
+// Columns k1 .. cend - 1 (k1 = k0 + NB), 32 per CTA: the panel's row exchanges, U12 = L11^-1 A12
+// (unit lower L11; a thread per column, its NB values in registers), and with `fused` also
+// A22 -= L21 U12 for the rows k1 .. rend - 1.  512 threads.
+template <int NB>
+__global__ void __launch_bounds__(kLuThreads) beam_lu_trailing_kernel(int n, int k0, int rend, int cend, int fused,
+                                                                      double* __restrict__ A,
+                                                                      const LuSwaps* __restrict__ swaps,
+                                                                      const int* __restrict__ status) {
+  constexpr int kRows = 64;  // rows of A22 per pass
+  constexpr int kQ = kRows / 16;
+  __shared__ double sl[NB][NB + 1];
+  __shared__ double sm[kRows][NB + 1];
+  __shared__ double su[NB][32 + 1];
+  if (status[0] != 0) return;
+  const int k1 = k0 + NB, c0 = k1 + blockIdx.x * 32, tid = threadIdx.x;
+  const int tx = tid & 31, ty = tid >> 5;  // ty: 0 .. 15
+  const int j = c0 + tx;
+  const bool on = j < cend;
+  constexpr int kMovedPerThread = kLuMaxPanel / 16;
+  const int nm = swaps->n_moved;
+  double mv[kMovedPerThread];
+#pragma unroll
+  for (int q = 0; q < kMovedPerThread; ++q) {
+    const int e = ty + 16 * q;
+    mv[q] = (on && e < nm) ? A[(int64_t)swaps->from[e] * n + j] : 0.0;
+  }
+  for (int k = ty; k < NB; k += 16) su[k][tx] = on ? A[(int64_t)swaps->src[k] * n + j] : 0.0;
+  for (int e = tid; e < NB * NB; e += kLuThreads) sl[e / NB][e % NB] = A[(int64_t)(k0 + e / NB) * n + k0 + e % NB];
+  __syncthreads();  // every source row of these columns has been read
+#pragma unroll
+  for (int q = 0; q < kMovedPerThread; ++q) {
+    const int e = ty + 16 * q;
+    if (on && e < nm) A[(int64_t)swaps->dest[e] * n + j] = mv[q];
+  }
+  __syncthreads();  // the moved rows of these columns are visible
+  double acc[kQ];
+  auto load_pass = [&](int r0) {
+    for (int e = tid; e < kRows * NB; e += kLuThreads) {
+      const int r = r0 + e / NB;
+      sm[e / NB][e % NB] = r < rend ? A[(int64_t)r * n + k0 + e % NB] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const int r = r0 + ty + 16 * q;
+      acc[q] = (on && r < rend) ? A[(int64_t)r * n + j] : 0.0;
+    }
+  };
+  if (fused) load_pass(k1);
+  if (ty == 0) {
+    double u[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) u[k] = su[k][tx];
+#pragma unroll
+    for (int k = 0; k < NB; ++k)
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        if (i > k) u[i] = fma(-sl[i][k], u[k], u[i]);
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      su[k][tx] = u[k];
+      if (on) A[(int64_t)(k0 + k) * n + j] = u[k];
+    }
+  }
+  if (!fused) return;
+  for (int r0 = k1; r0 < rend; r0 += kRows) {
+    __syncthreads();  // su and sm complete
+#pragma unroll 8
+    for (int k = 0; k < NB; ++k) {
+      const double uk = su[k][tx];
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) acc[q] = fma(-sm[ty + 16 * q][k], uk, acc[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const int r = r0 + ty + 16 * q;
+      if (on && r < rend) A[(int64_t)r * n + j] = acc[q];
+    }
+    if (r0 + kRows < rend) {
+      __syncthreads();  // sm free
+      load_pass(r0 + kRows);
+    }
   }
 }
 
-// columns j >= k0 + kLuPanel: the panel's row swaps in order, then U12 = L11^-1 A12 (unit lower
-// L11), one thread per column
-__global__ void beam_lu_swap_trsm_kernel(int n, int k0, double* __restrict__ A, const int* __restrict__ piv,
-                                         const int* __restrict__ status) {
+// A22 -= L21 U12 for the rows k1 .. rend - 1 and columns k1 .. cend - 1: a 32 x 32 tile per CTA
+// (32 x 8 threads, four rows each), L21 and U12 tiles staged in shared memory
+template <int NB>
+__global__ void __launch_bounds__(256) beam_lu_update_kernel(int n, int k0, int rend, int cend,
+                                                             double* __restrict__ A, const int* __restrict__ status) {
+  __shared__ double sl[32][NB + 1];
+  __shared__ double su[NB][32 + 1];
   if (status[0] != 0) return;
-  const int k1 = min(n, k0 + kLuPanel);
-  for (int j = k1 + blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    for (int k = k0; k < k1; ++k) {
-      const int p = piv[k - k0];
-      if (p != k) {
-        const double t = A[(int64_t)k * n + j];
-        A[(int64_t)k * n + j] = A[(int64_t)p * n + j];
-        A[(int64_t)p * n + j] = t;
-      }
-    }
-    for (int k = k0; k < k1; ++k) {
-      const double ukj = A[(int64_t)k * n + j];
-      for (int i = k + 1; i < k1; ++i) A[(int64_t)i * n + j] = fma(-A[(int64_t)i * n + k], ukj, A[(int64_t)i * n + j]);
-    }
-  }
-}
-
-// A22 -= L21 U12 for rows and columns >= k0 + kLuPanel: a 32 x 32 tile per CTA (32 x 8 threads,
-// four rows each), L21 and U12 tiles staged in shared memory
-__global__ void __launch_bounds__(256) beam_lu_update_kernel(int n, int k0, double* __restrict__ A,
-                                                             const int* __restrict__ status) {
-  __shared__ double sl[32][kLuPanel + 1];
-  __shared__ double su[kLuPanel][32 + 1];
-  if (status[0] != 0) return;
-  const int k1 = min(n, k0 + kLuPanel), w = k1 - k0;
+  const int k1 = k0 + NB;
   const int r0 = k1 + blockIdx.y * 32, c0 = k1 + blockIdx.x * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < 32 * kLuPanel; e += 256) {
-    const int r = e / kLuPanel, c = e % kLuPanel;
-    sl[r][c] = (r0 + r < n && c < w) ? A[(int64_t)(r0 + r) * n + k0 + c] : 0.0;
+  for (int e = threadIdx.x; e < 32 * NB; e += 256) {
+    const int r = e / NB, c = e % NB;
+    sl[r][c] = r0 + r < rend ? A[(int64_t)(r0 + r) * n + k0 + c] : 0.0;
     const int kr = e / 32, cc = e % 32;
-    su[kr][cc] = (kr < w && c0 + cc < n) ? A[(int64_t)(k0 + kr) * n + c0 + cc] : 0.0;
+    su[kr][cc] = c0 + cc < cend ? A[(int64_t)(k0 + kr) * n + c0 + cc] : 0.0;
   }
   __syncthreads();
   const int j = c0 + tx;
-  if (j >= n) return;
+  if (j >= cend) return;
+  double acc[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int r = ty + 8 * q, i = r0 + r;
-    if (i >= n) continue;
-    double a = A[(int64_t)i * n + j];
-    for (int k = 0; k < w; ++k) a = fma(-sl[r][k], su[k][tx], a);
-    A[(int64_t)i * n + j] = a;
+    const int i = r0 + ty + 8 * q;
+    acc[q] = i < rend ? A[(int64_t)i * n + j] : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < NB; ++k)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[q] = fma(-sl[ty + 8 * q][k], su[k][tx], acc[q]);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = r0 + ty + 8 * q;
+    if (i < rend) A[(int64_t)i * n + j] = acc[q];
   }
 }
 
-// back substitution with the upper factor, column oriented
-__global__ void __launch_bounds__(1024) beam_lu_backsub_kernel(int n, const double* __restrict__ A,
-                                                               double* __restrict__ b, const int* __restrict__ status) {
+// Back substitution with the upper factor (row k ends at column k + 2 kb), in blocks of 32
+// unknowns from the bottom, b in shared memory: one warp solves a block (lane i holds row i of its
+// triangle), then a thread per row above subtracts the block's columns, the last first; the
+// factor's values and reciprocals, which do not depend on x, are ready before the barrier.  One CTA
+// of 512 threads; bound by the chain of n quotients.
+__global__ void __launch_bounds__(kLuThreads) beam_lu_backsub_kernel(int n, int kb, const double* __restrict__ A,
+                                                                     double* __restrict__ b,
+                                                                     const int* __restrict__ status) {
+  __shared__ double sb[WN_BEAM_DENSE_MAX];
   if (status[0] != 0) return;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int k = n - 1; k >= 0; --k) {
-    if (tid == 0) b[k] /= A[(int64_t)k * n + k];
-    __syncthreads();
-    const double xk = b[k];
-    for (int i = tid; i < k; i += nt) b[i] = fma(-A[(int64_t)i * n + k], xk, b[i]);
-    __syncthreads();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < n; i += kLuThreads) sb[i] = b[i];
+  double u[32];  // warp 0: the block's triangle; the others: a row above it
+  auto load_row = [&](int i, int k0, int w, bool on) {  // n, k0 and w are even: 16-byte loads
+    const double2* __restrict__ row = reinterpret_cast<const double2*>(A + (int64_t)i * n + k0);
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const double2 v = (on && j < w) ? row[j / 2] : make_double2(0.0, 0.0);
+      u[j] = v.x;
+      u[j + 1] = v.y;
+    }
+  };
+  for (int k1 = n; k1 > 0; k1 -= 32) {
+    const int k0 = max(0, k1 - 32), w = k1 - k0;
+    const int lo = max(0, k0 - 2 * kb);  // rows whose factors reach the block
+    // warps 1 .. 15 take the rows above, 480 per pass
+    int i = lo + tid - 32;
+    if (warp == 0)
+      load_row(k0 + min(lane, w - 1), k0, w, true);
+    else
+      load_row(min(i, k0), k0, w, i < k0);
+    double diag = 1.0, rec = 1.0;  // the lane's diagonal entry
+    if (warp == 0) {
+#pragma unroll
+      for (int k = 0; k < 32; ++k)
+        if (lane == k && k < w) diag = u[k];
+      rec = 1.0 / diag;
+    }
+    __syncthreads();  // sb complete
+    if (warp == 0) {
+      const double x0 = lane < w ? sb[k0 + lane] : 0.0;
+      double x = x0;
+      // x_k / u_kk as a product with the reciprocal corrected once by its residual (the correctly
+      // rounded quotient wherever the reciprocal is, Markstein 1990): three operations of the chain
+      // instead of a division
+#pragma unroll
+      for (int k = 31; k >= 0; --k) {
+        const double q = x * rec;
+        const double xk = __shfl_sync(0xffffffffu, fma(fma(-q, diag, x), rec, q), k);
+        x = lane == k ? xk : lane < k ? fma(-u[k], xk, x) : x;
+      }
+      if (__any_sync(0xffffffffu, !isfinite(x))) {  // a reciprocal or product out of range: with divisions
+        x = x0;
+#pragma unroll 1
+        for (int k = w - 1; k >= 0; --k) {
+          if (lane == k) x /= diag;
+          const double xk = __shfl_sync(0xffffffffu, x, k);
+          if (lane < k) x = fma(-A[(int64_t)(k0 + lane) * n + k0 + k], xk, x);
+        }
+      }
+      if (lane < w) sb[k0 + lane] = x;
+    }
+    __syncthreads();  // the block's unknowns are final
+    if (warp != 0)
+      for (; i < k0; i += kLuThreads - 32) {
+        if (i >= lo + kLuThreads - 32) load_row(i, k0, w, true);
+        double x = sb[i];
+#pragma unroll
+        for (int k = 31; k >= 0; --k)
+          if (k < w) x = fma(-u[k], sb[k0 + k], x);
+        sb[i] = x;
+      }
   }
+  __syncthreads();
+  for (int i = tid; i < n; i += kLuThreads) b[i] = sb[i];
 }
 
 }  // namespace wn
@@ -396,9 +626,11 @@ struct Beam {
   DArray<double> fe, ke, K, dinv;
   // BiCGStab workspace
   DArray<double> r, rh, p, v, s, t, y, z, x, part;
-  // dense LU workspace (small frames)
+  // dense LU workspace (small frames) and the matrix's half bandwidth in DOFs
   DArray<double> dense;
   DArray<int> dstat;
+  DArray<LuSwaps> dswaps;
+  int half_band = 0;
   bool assembled = false;
 };
 
@@ -529,6 +761,10 @@ int wn_beam_create(int64_t n_nodes, int64_t n_el, const double* nodes, const int
   std::vector<int64_t> iptr;
   int rc = build_beam_pattern(n_nodes, n_el, elements, *b, b->h_rp, b->h_ci, brow, diag, gptr, gsrc, iptr, iea);
   const int64_t n = n_nodes * 6;
+  int64_t apart = 0;  // nodes, between the ends of a beam
+  if (rc == 0)
+    for (int64_t e = 0; e < n_el; ++e) apart = std::max<int64_t>(apart, std::abs(elements[2 * e] - elements[2 * e + 1]));
+  b->half_band = (int)std::min<int64_t>(6 * apart + 5, WN_BEAM_DENSE_MAX);
   rc = rc ? rc : b->nodes.upload(nodes, n_nodes * 3);
   rc = rc ? rc : b->el.upload(elements, n_el * 2);
   rc = rc ? rc : b->props.upload(props, n_el * 6);
@@ -674,6 +910,50 @@ int wn_beam_linear_system(void* h, void** out) {
                           any ? fixed.data() : nullptr, out);
 }
 
+}  // extern "C"
+
+// one panel of dense_lu of NB columns, rows in registers (RPT per thread)
+template <int NB, int RPT>
+static void lu_panel(Beam* b, double* d_x, int n, int k0, int rend, int cend, cudaStream_t st) {
+  const int m = rend - k0, k1 = std::min(n, k0 + NB);
+  const int threads = std::min(kLuThreads, std::max(64, ((m + RPT - 1) / RPT + 31) / 32 * 32));
+  beam_lu_panel_kernel<NB, RPT><<<1, threads, 0, st>>>(n, k0, rend, b->dense.p, d_x, b->dswaps.p, b->dstat.p);
+  if (cend <= k1) return;
+  const int strips = (cend - k1 + 31) / 32, rows = rend - k1;
+  const int fused = rows <= kLuFuseRows;
+  beam_lu_trailing_kernel<NB><<<strips, kLuThreads, 0, st>>>(n, k0, rend, cend, fused, b->dense.p, b->dswaps.p,
+                                                             b->dstat.p);
+  if (!fused)
+    beam_lu_update_kernel<NB><<<dim3((unsigned)strips, (unsigned)((rows + 31) / 32)), 256, 0, st>>>(
+        n, k0, rend, cend, b->dense.p, b->dstat.p);
+}
+
+// LU of the dense copy and the solve (d_x: right-hand side in, solution out).  The widest panel
+// whose rows fit the registers of one CTA: 32 columns up to 512 rows (64 registers a thread hold
+// one row), then 16 columns x 2 rows, 8 x 4 and 8 x 6 (3,072 rows, WN_BEAM_DENSE_MAX); the band
+// decides, not n.
+static int dense_lu(Beam* b, double* d_x, int n, cudaStream_t st) {
+  const int kb = std::min(n - 1, b->half_band);
+  const int64_t tall = std::min<int64_t>(n, (int64_t)kb + kLuMaxPanel);
+  const int nb = tall <= kLuThreads ? 32 : tall <= 2 * kLuThreads ? 16 : 8;
+  for (int k0 = 0; k0 < n; k0 += nb) {
+    const int k1 = std::min(n, k0 + nb), rend = std::min(n, k1 + kb), cend = std::min(n, k1 + 2 * kb);
+    if (nb == 32)
+      lu_panel<32, 1>(b, d_x, n, k0, rend, cend, st);
+    else if (nb == 16)
+      lu_panel<16, 2>(b, d_x, n, k0, rend, cend, st);
+    else if (tall <= 4 * kLuThreads)
+      lu_panel<8, 4>(b, d_x, n, k0, rend, cend, st);
+    else
+      lu_panel<8, 6>(b, d_x, n, k0, rend, cend, st);
+  }
+  beam_lu_backsub_kernel<<<1, kLuThreads, 0, st>>>(n, kb, b->dense.p, d_x, b->dstat.p);
+  WN_CUDA(cudaGetLastError());
+  return 0;
+}
+
+extern "C" {
+
 int wn_beam_solve_device(void* h, const double* d_b, double* d_x, int method, double rtol, int max_iter, int* iters,
                          double* rel_res, uintptr_t stream) {
   WN_REQUIRE(h && d_b && d_x && rtol > 0 && max_iter > 0 && method >= 0 && method <= 2, WN_EINVAL,
@@ -687,23 +967,13 @@ int wn_beam_solve_device(void* h, const double* d_b, double* d_x, int method, do
     WN_REQUIRE(n <= WN_BEAM_DENSE_MAX, WN_ETOOBIG, "wn_beam_solve_device: dense LU limited to %d DOFs",
                WN_BEAM_DENSE_MAX);
     WN_CHECK(b->dense.alloc(n * n));
-    WN_CHECK(b->dstat.alloc(1 + kLuPanel));  // [0] status, [1..] the current panel's pivots
+    WN_CHECK(b->dstat.alloc(1));
+    WN_CHECK(b->dswaps.alloc(1));
     WN_CUDA(cudaMemsetAsync(b->dense.p, 0, n * n * sizeof(double), st));
     WN_CUDA(cudaMemsetAsync(b->dstat.p, 0, sizeof(int), st));
     beam_dense_kernel<<<grid_for(n, 1, 256, 8), 256, 0, st>>>(b->n_nodes, b->rp.p, b->ci.p, b->K.p, b->dense.p);
     WN_CUDA(cudaMemcpyAsync(d_x, d_b, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    const int ni = (int)n;
-    int* piv = b->dstat.p + 1;
-    for (int k0 = 0; k0 < ni; k0 += kLuPanel) {
-      beam_lu_panel_kernel<<<1, 1024, 0, st>>>(ni, k0, b->dense.p, d_x, piv, b->dstat.p);
-      const int rest = ni - std::min(ni, k0 + kLuPanel);
-      if (rest > 0) {
-        beam_lu_swap_trsm_kernel<<<(rest + 127) / 128, 128, 0, st>>>(ni, k0, b->dense.p, piv, b->dstat.p);
-        const unsigned tiles = (unsigned)((rest + 31) / 32);
-        beam_lu_update_kernel<<<dim3(tiles, tiles), 256, 0, st>>>(ni, k0, b->dense.p, b->dstat.p);
-      }
-    }
-    beam_lu_backsub_kernel<<<1, 1024, 0, st>>>(ni, b->dense.p, d_x, b->dstat.p);
+    WN_CHECK(dense_lu(b, d_x, (int)n, st));
     WN_CUDA(cudaGetLastError());
     int stat = 0;
     WN_CUDA(cudaMemcpyAsync(&stat, b->dstat.p, sizeof(int), cudaMemcpyDeviceToHost, st));
