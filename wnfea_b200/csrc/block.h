@@ -1,25 +1,30 @@
-// Multi-right-hand-side (batched) PCG workspace: up to kBatch load cases solved together
-// against one assembled matrix and one AMG hierarchy.
+// Multi-right-hand-side (batched) PCG workspace: up to kBatch (8, 16 or 32) load cases solved
+// together against one assembled matrix and one AMG hierarchy.
 //
 // Layout: a batched vector of n scalar DOFs is n x kBatch, DOF-major with the kBatch load
-// cases of one DOF contiguous (element (i, j) at i * kBatch + j; 128 B per DOF in FP32, 256 B
-// in FP64).  A block row of the matrix is handled by 8 lanes, each owning 4 consecutive load
-// cases, so every matrix block is read once per product for all kBatch cases.
+// cases of one DOF contiguous (element (i, j) at i * kBatch + j).  A block row of the matrix is
+// handled by 8 lanes, each owning kBatch / 8 load cases, so every matrix block is read once per
+// product for all kBatch cases.
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <vector>
 
 #include "amg.h"
 #include "device_array.h"
+#include "wnfea_cuda.h"
 
 namespace wn {
 
-constexpr int kBatch = 32;
+struct Solid;  // solid.h
+
+constexpr int kMaxBatch = 32;
 
 // per-load-case PCG state (device)
-struct BlockScalars {
+template <int kBatch>
+struct BlockScalarsT {
   double rz[kBatch];      // r . z of the current iteration
   double alpha[kBatch];   // step of the current iteration (0 for finished cases)
   double beta[kBatch];    // p = z + beta p of the next iteration (0 for finished cases)
@@ -35,27 +40,35 @@ struct BlockScalars {
   int max_iter;
 };
 
+// Vectors of a V-cycle level.  The finest level's right-hand side and result are the PCG's, and r, d
+// and d2 belong to Chebyshev steps beyond the first: left out where nothing reads them (at 32 cases
+// a fine vector of a million DOFs is 130 MB in FP32).
 template <typename T>
 struct BatchLevelVecs {
   DArray<T> b, x, x2, r, d, d2, res;
-  int alloc(int64_t n) {
-    WN_CHECK(b.alloc(n));
+  int alloc(int64_t n, bool finest, int degree) {
+    if (!finest) {
+      WN_CHECK(b.alloc(n));
+      WN_CHECK(x2.alloc(n));
+    }
     WN_CHECK(x.alloc(n));
-    WN_CHECK(x2.alloc(n));
-    WN_CHECK(r.alloc(n));
-    WN_CHECK(d.alloc(n));
-    WN_CHECK(d2.alloc(n));
     WN_CHECK(res.alloc(n));
+    if (degree > 1) {
+      WN_CHECK(r.alloc(n));
+      WN_CHECK(d.alloc(n));
+      WN_CHECK(d2.alloc(n));
+    }
     return 0;
   }
 };
 
-struct BlockWork {
+template <int kBatch>
+struct BlockWorkT {
   int64_t n = 0;  // scalar DOFs of the fine level
   static constexpr int kMaxParts = 148 * 16;
   int npA = 0, npB = 0, npC = 0;
   DArray<double> partA, partB, partC;  // kMaxParts x kBatch
-  DArray<BlockScalars> scal;           // [0] inner PCG, [1] outer column norms
+  DArray<BlockScalarsT<kBatch>> scal;  // [0] inner PCG, [1] outer column norms
   DArray<double> rtol_cols;            // kBatch inner targets
   std::vector<double> h_rtol;
   // outer refinement: F, U = U + Ulo (double-double), R = F - K U
@@ -77,7 +90,7 @@ struct BlockWork {
   DArray<float> cb32, cx32;
   DArray<double> cb64, cx64;
   uint64_t hierarchy_id = 0;        // the AmgHierarchy the level vectors were sized for
-  // x-tiles of the fine level (block_solver.cu build_x_tiles): runs of rows whose blocks name at
+  // x-tiles of the fine level (block_batch.cuh build_x_tiles): runs of rows whose blocks name at
   // most 256 columns; per tile its sorted columns, per block its column's index among them
   DArray<int32_t> xt_rows, xt_col_ptr, xt_cols;
   DArray<uint8_t> xt_lcol;
@@ -85,15 +98,57 @@ struct BlockWork {
   bool xt_tried = false;
   GraphCache graphs[2][3];          // [V-cycle precision 0 fp64 / 1 fp32][preconditioner]
   int64_t launches = 0;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  cudaStream_t own = nullptr;
-  ~BlockWork() {
+  ~BlockWorkT() {
     for (auto& a : graphs)
       for (auto& g : a) g.reset();
+  }
+};
+
+// the batched solver of one handle
+struct BlockSet {
+  // the fine level's rows as the row kernels of 2 and 3 CTAs per SM take them (batch_order)
+  DArray<int32_t> order[2];
+  std::unique_ptr<BlockWorkT<8>> w8;
+  std::unique_ptr<BlockWorkT<16>> w16;
+  std::unique_ptr<BlockWorkT<32>> w32;
+  template <int W>
+  std::unique_ptr<BlockWorkT<W>>& width() {
+    if constexpr (W == 8)
+      return w8;
+    else if constexpr (W == 16)
+      return w16;
+    else
+      return w32;
+  }
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaStream_t own = nullptr;
+  ~BlockSet() {
+    w8.reset();
+    w16.reset();
+    w32.reset();
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (own) cudaStreamDestroy(own);
   }
 };
+
+struct BatchResult {
+  int iterations = 0, outer = 0, status = 0;
+  int case_iters[kMaxBatch] = {};
+  int case_status[kMaxBatch] = {};
+  double case_rel[kMaxBatch] = {};
+  int64_t launches = 0;
+};
+
+// load cases j0 .. j0 + m - 1 (m <= W) of the row-major n x n_rhs F into U (block_batch.cuh)
+template <int W>
+int solve_batch(Solid* s, const double* F, double* U, int n_rhs, int j0, int m, const wn_solve_params& prm,
+                BatchResult& res, cudaStream_t st);
+template <>
+int solve_batch<8>(Solid*, const double*, double*, int, int, int, const wn_solve_params&, BatchResult&, cudaStream_t);
+template <>
+int solve_batch<16>(Solid*, const double*, double*, int, int, int, const wn_solve_params&, BatchResult&, cudaStream_t);
+template <>
+int solve_batch<32>(Solid*, const double*, double*, int, int, int, const wn_solve_params&, BatchResult&, cudaStream_t);
 
 }  // namespace wn

@@ -15,7 +15,7 @@ namespace wn {
 
 struct AmgHierarchy;  // amg.h
 struct SolverWork;    // solver.cu
-struct BlockWork;     // block.h
+struct BlockSet;      // block.h
 
 constexpr int kStreamStatusWord = 8;
 
@@ -62,7 +62,7 @@ struct Solid {
   uint64_t values_version = 0;  // bumped whenever the matrix values change (the FP16 pack's tag)
   std::unique_ptr<AmgHierarchy> amg;
   std::unique_ptr<SolverWork> work;
-  std::unique_ptr<BlockWork> bwork;
+  std::unique_ptr<BlockSet> batch;
   // host-buffer solve: device copies of F / u and a page-locked staging buffer (2 n), kept
   // between calls so that a call neither allocates nor copies from pageable memory; one event
   // per staged chunk of the result (its copy out of the staging buffer waits for that chunk only)
