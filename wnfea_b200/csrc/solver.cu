@@ -292,8 +292,10 @@ __global__ void __launch_bounds__(kThreads, (BS == 3) ? kMinBlocks : 1) k_post_f
       const T r0 = dinv[i] * (b[i] - pick<BS>(acc, lane));
       const T d0 = r0 * inv_theta;
       const T xn = x[i] + d0;
-      r[i] = r0;
-      d[i] = d0;
+      if (r) {  // a Chebyshev step follows
+        r[i] = r0;
+        d[i] = d0;
+      }
       x2[i] = xn;
       if (part) dot += (double)b[i] * (double)xn;
     }
@@ -885,8 +887,10 @@ struct EpiPostFirst {
     const T r0 = p.di * (p.bi - t);
     const T d0 = r0 * inv_theta;
     const T xn = p.xi + d0;
-    r[i] = r0;
-    d[i] = d0;
+    if (r) {  // a Chebyshev step follows
+      r[i] = r0;
+      d[i] = d0;
+    }
     x2[i] = SC ? p.si * xn : xn;
     return want_dot ? (double)p.bi * (double)xn : 0.0;
   }
@@ -1076,12 +1080,125 @@ static bool launch_stream_rows(const StreamMat& m, XF xf, EPI epi, double* part,
   return true;
 }
 
-// y = M x or y += M x for a transfer operator: streamed from its pack when it has one, else the
-// register row kernel
+// ---------------------------------------------------------------------------------------
+// 6-row block matrices with long rows: W warps per block row (8 / W rows per CTA)
+// ---------------------------------------------------------------------------------------
+// The coarse levels of a solid with little surface have rows of 100 to 500 blocks and few of them
+// (the 162,000-element block: 2,116 rows of 413 blocks, then 385 of 343), and a restriction's rows are
+// as long.  A warp per row walks such a row in up to 16 dependent rounds of 32 blocks while most
+// of the SMs' warps have no row, and a streamed tile of 256 blocks holds one row, which one of its
+// eight consumer warps computes.  Here a row is spread over W warps, a lane takes its blocks W x 32
+// apart, and its first block's values and column -- which no kernel of the solve writes -- are
+// loaded before griddepcontrol.wait, while the previous kernel finishes.
+
+template <int BC, int W, typename T, typename XF, typename EPI>
+__global__ void __launch_bounds__(kThreads) k_team_rows(int64_t n_rows, const int32_t* __restrict__ rp,
+                                                        const int32_t* __restrict__ ci, const T* __restrict__ av,
+                                                        XF xf, EPI epi, double* __restrict__ part,
+                                                        const PcgScalars* __restrict__ S) {
+  constexpr int BR = 6, NB = BR * BC, R = (kThreads / 32) / W;  // rows per CTA
+  __shared__ T sums[2][kThreads / 32][BR];
+  __shared__ double sh[kThreads / 32];
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, team = warp / W, tl = threadIdx.x % (32 * W);
+  T v[NB];
+  int32_t col = 0;
+  auto load = [&](int32_t b) {
+    col = __ldg(ci + b);
+    BlockLoad<T, NB>::load(av + (int64_t)b * NB, v);
+  };
+  int64_t row = (int64_t)blockIdx.x * R + team;
+  int32_t b = 0, e = 0;
+  auto begin_row = [&]() {
+    b = e = 0;
+    if (row < n_rows) {
+      b = __ldg(rp + row) + tl;
+      e = __ldg(rp + row + 1);
+      if (b < e) load(b);
+    }
+  };
+  begin_row();
+  pdl_wait();
+  if (*(volatile const int*)&S->done) return;
+  double dot = 0.0;
+  int turn = 0;
+  for (int64_t base = (int64_t)blockIdx.x * R; base < n_rows; base += (int64_t)gridDim.x * R, turn ^= 1) {
+    // the row's own operands, by the lanes that will store its DOFs
+    const bool owner = tl < BR && row < n_rows;
+    typename EPI::Pre pre{};
+    if (owner) pre = epi.load(row * BR + tl);
+    T acc[BR];
+#pragma unroll
+    for (int r = 0; r < BR; ++r) acc[r] = T(0);
+    while (b < e) {
+      T x[BC];
+#pragma unroll
+      for (int c = 0; c < BC; ++c) x[c] = xf((int64_t)col * BC + c);
+#pragma unroll
+      for (int r = 0; r < BR; ++r)
+#pragma unroll
+        for (int c = 0; c < BC; ++c) acc[r] = fma(v[r * BC + c], x[c], acc[r]);
+      b += 32 * W;
+      if (b < e) load(b);
+    }
+    const int64_t mine = row;
+    row += (int64_t)gridDim.x * R;
+    begin_row();  // the next row's first blocks are on their way during the reduction
+    const T sum = group_sum_transposed<BR, 32>(acc, lane);
+    if ((lane & 3) == 0 && (lane >> 2) < BR) sums[turn][warp][lane >> 2] = sum;
+    __syncthreads();
+    if (owner) {
+      T t = T(0);
+#pragma unroll
+      for (int w = 0; w < W; ++w) t += sums[turn][team * W + w][tl];
+      dot += epi.store(mine * BR + tl, pre, t);
+    }
+  }
+  if (part) write_part(dot, part, sh);
+}
+
+// Warps per row for a matrix of 6-row blocks by its mean blocks per row, 0: the streamed or
+// warp-per-row kernels.  Measured (FP32, event-timed, warp-per-row or streamed -> teams):
+//   no pack: 413 blocks, 130 MB  43 -> 33 us; 343, 20 MB  21 -> 12 us; restrictions of 27 / 2.5 MB
+//            45 -> 14 and 26 -> 10 us;
+//   packed:  243, 76 MB  38 -> 24 us; 100, 30 MB  16 -> 15 us; but 134, 300 MB  76 -> 78 us and 105
+//            (6x3), 140 MB  33 -> 42 us: a pack of more than L2's share streams better until a row
+//            fills most of a tile.
+static int team_width(int64_t n_rows, int64_t nnzb, int block_bytes, bool packed) {
+  if (n_rows <= 0) return 0;
+  const double avg = (double)nnzb / (double)n_rows;
+  const bool big = (double)nnzb * block_bytes > 48e6;
+  if (avg < (packed ? (big ? 192.0 : 96.0) : 64.0)) return 0;
+  return avg >= 160.0 ? 8 : 4;
+}
+
+template <int BC, typename T, typename XF, typename EPI>
+static bool launch_team_rows(int64_t n_rows, int64_t nnzb, bool packed, const int32_t* rp, const int32_t* ci,
+                             const T* av, XF xf, EPI epi, double* part, const PcgScalars* S, cudaStream_t st,
+                             int* grid_out) {
+  const int w = team_width(n_rows, nnzb, 6 * BC * (int)sizeof(T), packed);
+  if (w == 0) return false;
+  auto go = [&](auto kern, int rows_per_cta) {
+    const int g = resident_grid(kern, kThreads, (n_rows + rows_per_cta - 1) / rows_per_cta);
+    if (grid_out) *grid_out = g;
+    return launch_pdl(kern, g, kThreads, 0, st, n_rows, rp, ci, av, xf, epi, part, S) == cudaSuccess;
+  };
+  const bool ok = w == 8 ? go(k_team_rows<BC, 8, T, XF, EPI>, 1) : go(k_team_rows<BC, 4, T, XF, EPI>, 2);
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
+// y = M x or y += M x for a transfer operator: long rows by teams of warps, else streamed from its
+// pack when it has one, else the register row kernel
 // (SC: (M x)_i scaled by ys_i -- the FP16 V-cycle's prolongation into its scaled fine level)
 template <int BR, int BC, typename T, bool SC = false>
 static void level_spmv(const DevBsr& M, const StreamMat& Ms, const T* vals, const T* x, T* y, int accumulate,
                        PcgScalars* S, cudaStream_t st, const T* ys = nullptr) {
+  if constexpr (BR == 6 && !SC) {
+    if (launch_team_rows<BC, T>(M.n_rows, M.nnzb, Ms.packed, M.rp.p, M.ci.p, vals, XLoad<T, T>{x},
+                                EpiLevel<T, false>{y, accumulate, nullptr}, nullptr, S, st, nullptr))
+      return;
+  }
   if constexpr (BR == 6 && BC == 6) {  // short rows (the prolongations): 8 lanes per row
     if (M.nnzb < 16 * M.n_rows) {
       if (launch_stream_rows<T, 6, 6, XLoad<T, T>, EpiLevel<T, SC>, StreamShort66<T>>(
@@ -1243,6 +1360,10 @@ static int vcycle(Solid* s, AmgHierarchy& H, SolverWork& W, int lvl, const T* b,
         half_failed = half_failed || !ok;
         return true;
       } else {
+        if constexpr (BS == 6) {
+          if (launch_team_rows<BS, T>(nr, lvl == 0 ? s->nnzb : L.A.nnzb, stream, rp, ci, av, xf, epi, prt, S, st, gout))
+            return true;
+        }
         return stream && launch_stream_rows<T, BS, BS>(Am, xf, epi, prt, S, st, gout);
       }
     };
@@ -1296,16 +1417,17 @@ static int vcycle(Solid* s, AmgHierarchy& H, SolverWork& W, int lvl, const T* b,
     // post-smoothing: result in `out`
     double* part_last = (deg == 1) ? part : nullptr;
     int gpf = 0;
-    EpiPostFirst<T, SC> epi_post{b, dinv, it, V.x.p, out, V.r.p, V.d.p, part_last != nullptr};
+    T* r_post = deg == 1 ? nullptr : V.r.p;
+    EpiPostFirst<T, SC> epi_post{b, dinv, it, V.x.p, out, r_post, V.d.p, part_last != nullptr};
     epi_post.os = deg == 1 ? os : nullptr;
     if (!rows(XLoad<T, T>{V.x.p}, epi_post, part_last, &gpf)) {
       gpf = rg(k_post_first<BS, T>);
-      k_post_first<BS, T><<<gpf, kThreads, 0, st>>>(nr, rp, ci, av, sd, b, dinv, it, V.x.p, out, V.r.p, V.d.p,
+      k_post_first<BS, T><<<gpf, kThreads, 0, st>>>(nr, rp, ci, av, sd, b, dinv, it, V.x.p, out, r_post, V.d.p,
                                                      part_last, S);
     }
     if (part_last) W.npA = gpf;
     W.launches++;
-    note(W, st, "post_smooth", lvl, Ab + 6 * Vb);
+    note(W, st, "post_smooth", lvl, Ab + (deg == 1 ? 4 : 6) * Vb);
     din = V.d.p;
     dout = V.d2.p;
     for (int k = 1; k < deg; ++k) {
