@@ -35,6 +35,7 @@
 #include "common.cuh"
 #include "eft.cuh"
 #include "kernels.h"
+#include "small_solve.h"
 #include "solid.h"
 #include "spmv.cuh"
 #include "solver.h"
@@ -1623,6 +1624,10 @@ static int pcg_iteration(Solid* s, SolverWork& W, int precond, int k, PcgScalars
 template <typename TK, typename TM>
 static int pcg_solve(Solid* s, SolverWork& W, int mode, const TK* b, double rtol, int max_iter, int precond,
                      int chunk, int use_graph, PcgScalars* S, cudaStream_t st, PcgScalars* hS) {
+  if constexpr (std::is_same<TK, double>::value) {
+    const int rc = small_pcg<TM>(s, W, b, rtol, max_iter, precond, S, st, hS);
+    if (rc != 1) return rc;
+  }
   PcgBufs<TK, TM> B = pcg_bufs<TK, TM>(s, W);
   WN_CUDA(cudaMemsetAsync(B.p0, 0, W.n * sizeof(TK), st));  // iteration 0: p = z + 0 * p_old
   WN_CUDA(cudaMemsetAsync(B.p1, 0, W.n * sizeof(TK), st));
