@@ -81,20 +81,38 @@ __global__ void ks_inv_diag(DMat A, double* __restrict__ dinv) {
 }
 
 // y = A x with the host builder's order: per row DOF, per block the row's dot product, added in
-// block order
-__global__ void ks_spmv_rows(DMat A, const double* __restrict__ x, double* __restrict__ y) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < A.n_rows * A.br;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t / A.br;
-    const int r = (int)(t - i * A.br);
+// block order.  A warp per block row, a lane per block for the dot products; they go through
+// shared memory to the lanes that add them up in order.  (A thread per row DOF reads a row's values
+// one after the other, each from another sector: 188 us per product on a 42,000-node matrix and its
+// levels against 32.)
+template <int BS>
+__global__ void __launch_bounds__(kT) ks_spmv_rows(DMat A, const double* __restrict__ x, double* __restrict__ y) {
+  __shared__ double sums[kT / 32][32][BS + 1];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < A.n_rows; i += nw) {
+    const int32_t k0 = A.rp[i], k1 = A.rp[i + 1];
     double acc = 0.0;
-    for (int32_t k = A.rp[i]; k < A.rp[i + 1]; ++k) {
-      const double* xx = x + (int64_t)A.ci[k] * A.bc;
-      double s = 0.0;
-      for (int c = 0; c < A.bc; ++c) s += A.at(k, r, c) * xx[c];
-      acc += s;
+    for (int32_t base = k0; base < k1; base += 32) {
+      const int32_t k = base + lane;
+      if (k < k1) {
+        const double* xx = x + (int64_t)A.ci[k] * BS;
+#pragma unroll
+        for (int r = 0; r < BS; ++r) {
+          double s = 0.0;
+#pragma unroll
+          for (int c = 0; c < BS; ++c) s = fma(A.at(k, r, c), xx[c], s);
+          sums[w][lane][r] = s;
+        }
+      }
+      __syncwarp();
+      if (lane < BS) {
+        const int n = min(32, k1 - base);
+        for (int q = 0; q < n; ++q) acc += sums[w][q][lane];
+      }
+      __syncwarp();
     }
-    y[t] = acc;
+    if (lane < BS) y[i * BS + lane] = acc;
   }
 }
 
@@ -136,13 +154,64 @@ __global__ void ks_block_norms(DMat A, double* __restrict__ nrm) {
   }
 }
 
+// Strength of connection, the host builder's aggregate_norms: block (i, j) is strong when its norm
+// reaches theta sqrt(norm_ii norm_jj).  One byte per block and per row (any strong) go to the host
+// instead of the norms; the same products, roots and comparisons, so the same bits.
+__global__ void ks_diag_norms(int64_t n_rows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                              const double* __restrict__ nrm, double* __restrict__ dn) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rows; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t k = find_col(ci, rp[i], rp[i + 1], (int32_t)i);
+    dn[i] = k >= 0 ? nrm[k] : 0.0;
+  }
+}
+
+__global__ void ks_strong(int64_t n_rows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                          const double* __restrict__ nrm, const double* __restrict__ dn, double theta,
+                          uint8_t* __restrict__ strong, uint8_t* __restrict__ has_strong) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n_rows; i += nw) {
+    bool any = false;
+    for (int32_t k = rp[i] + lane; k < rp[i + 1]; k += 32) {
+      const int32_t j = ci[k];
+      const bool is = j != i && nrm[k] > 0.0 && nrm[k] >= __dmul_rn(theta, __dsqrt_rn(__dmul_rn(dn[i], dn[j])));
+      strong[k] = is;
+      any = any || is;
+    }
+    any = __any_sync(0xffffffffu, any);
+    if (lane == 0) has_strong[i] = any;
+  }
+}
+
+// pass 2 of the aggregation: an unaggregated row joins the aggregate of its strongest aggregated
+// strong neighbour (the first of the strongest)
+__global__ void ks_join(int64_t n_rows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                        const double* __restrict__ nrm, const uint8_t* __restrict__ strong,
+                        const int32_t* __restrict__ agg, int32_t* __restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rows; i += (int64_t)gridDim.x * blockDim.x) {
+    int32_t a = agg[i];
+    if (a < 0) {
+      double best = -1.0;
+      for (int32_t k = rp[i]; k < rp[i + 1]; ++k)
+        if (strong[k] && agg[ci[k]] >= 0 && nrm[k] > best) {
+          best = nrm[k];
+          a = agg[ci[k]];
+        }
+    }
+    out[i] = a;
+  }
+}
+
 // ---------------------------------------------------------------------------------------
 // smoothed prolongator P = P_tent - w D^-1 A P_tent (row i: bs x 6 blocks at the aggregates of
 // i and of its neighbours)
 // ---------------------------------------------------------------------------------------
-// one warp per row: the sorted unique aggregates of the row (count, or columns when out_ci)
-__global__ void ks_p_pattern(DMat A, const int32_t* __restrict__ agg, int smooth, int32_t* __restrict__ cnt,
-                             const int32_t* __restrict__ rp_out, int32_t* __restrict__ ci_out, int* __restrict__ err) {
+// one warp per row: the sorted unique aggregates of the row (count, or columns when out_ci).  The
+// row's candidates are taken 32 at a time: a value that is not in the list yet is appended by its
+// first lane; the ranks are then counted within the list.
+__global__ void __launch_bounds__(kT) ks_p_pattern(DMat A, const int32_t* __restrict__ agg, int smooth,
+                                                   int32_t* __restrict__ cnt, const int32_t* __restrict__ rp_out,
+                                                   int32_t* __restrict__ ci_out, int* __restrict__ err) {
   __shared__ int32_t buf[kT / 32][kWarpBuf];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int32_t* b = buf[w];
@@ -154,105 +223,128 @@ __global__ void ks_p_pattern(DMat A, const int32_t* __restrict__ agg, int smooth
       if (lane == 0) *err = 1;
       continue;
     }
-    for (int p = lane; p < m; p += 32) b[p] = p == 0 ? agg[i] : agg[A.ci[k0 + p - 1]];
-    __syncwarp();
-    // unique values: first occurrence of each value >= 0; rank = distinct values below it
-    int local = 0;
-    for (int p = lane; p < m; p += 32) {
-      const int32_t v = b[p];
-      bool first = v >= 0;
-      for (int q = 0; q < p && first; ++q) first = b[q] != v;
-      if (!first) continue;
-      ++local;
-      if (ci_out) {
+    int n = 0;  // distinct values so far
+    for (int base = 0; base < m; base += 32) {
+      const int p = base + lane;
+      const int32_t v = p >= m ? -1 : p == 0 ? agg[i] : agg[A.ci[k0 + p - 1]];
+      const unsigned same = __match_any_sync(0xffffffffu, v);
+      bool fresh = v >= 0 && (__ffs(same) - 1) == lane;
+      for (int q = 0; q < n && fresh; ++q) fresh = b[q] != v;
+      const unsigned add = __ballot_sync(0xffffffffu, fresh);
+      if (fresh) b[n + __popc(add & ((1u << lane) - 1))] = v;
+      n += __popc(add);
+      __syncwarp();
+    }
+    if (ci_out)
+      for (int p = lane; p < n; p += 32) {
+        const int32_t v = b[p];
         int rank = 0;
-        for (int q = 0; q < m; ++q) {
-          const int32_t u = b[q];
-          if (u < 0 || u >= v) continue;
-          bool fu = true;
-          for (int z = 0; z < q && fu; ++z) fu = b[z] != u;
-          rank += fu;
-        }
+        for (int q = 0; q < n; ++q) rank += b[q] < v;
         ci_out[rp_out[i] + rank] = v;
       }
-    }
-    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-    if (lane == 0 && cnt) cnt[i] = local;
+    if (lane == 0 && cnt) cnt[i] = n;
     __syncwarp();
   }
 }
 
-// values of the P pattern (thread per block); nzflag[k] = 1 if the block is not all zero
+// values of the P pattern; nzflag[k] = 1 if the block is not all zero.  A warp per block of P: its
+// lanes look for the row's neighbours in the aggregate, 32 at a time; those found are added in order,
+// a lane per entry of the block (two for the first lanes of a 6x6 one).
 template <int BS>
-__global__ void ks_p_values(DMat A, const int32_t* __restrict__ agg, const double* __restrict__ qnode,
-                            const double* __restrict__ dinv, double w, const int32_t* __restrict__ prow,
-                            const int32_t* __restrict__ pci, int64_t nnz, double* __restrict__ pv,
-                            uint8_t* __restrict__ nzflag) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nnz; q += (int64_t)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(kT) ks_p_values(DMat A, const int32_t* __restrict__ agg,
+                                                  const double* __restrict__ qnode, const double* __restrict__ dinv,
+                                                  double w, const int32_t* __restrict__ prow,
+                                                  const int32_t* __restrict__ pci, int64_t nnz,
+                                                  double* __restrict__ pv, uint8_t* __restrict__ nzflag) {
+  constexpr int NE = BS * 6, EL = (NE + 31) / 32;  // entries of a block, of a lane
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t q = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; q < nnz; q += nw) {
     const int64_t i = prow[q];
     const int32_t a = pci[q];
-    double s[BS * 6];
+    double s[EL], f[EL];
+    int r[EL], t[EL];
+    const bool own = agg[i] == a;
 #pragma unroll
-    for (int e = 0; e < BS * 6; ++e) s[e] = 0.0;
-    if (agg[i] == a) {
-#pragma unroll
-      for (int e = 0; e < BS * 6; ++e) s[e] += qnode[i * BS * 6 + e];
+    for (int u = 0; u < EL; ++u) {
+      const int e = min(lane + 32 * u, NE - 1);
+      r[u] = e / 6;
+      t[u] = e % 6;
+      s[u] = own ? qnode[i * NE + e] : 0.0;
+      f[u] = -w * dinv[i * BS + r[u]];
     }
     if (w != 0.0) {
-      for (int32_t k = A.rp[i]; k < A.rp[i + 1]; ++k) {
-        const int32_t j = A.ci[k];
-        if (agg[j] != a) continue;
-        const double* qj = qnode + (int64_t)j * BS * 6;
+      const int32_t k1 = A.rp[i + 1];
+      for (int32_t base = A.rp[i]; base < k1; base += 32) {
+        const int32_t j_mine = base + lane < k1 ? A.ci[base + lane] : -1;
+        unsigned hit = __ballot_sync(0xffffffffu, j_mine >= 0 && agg[max(j_mine, 0)] == a);
+        while (hit) {
+          const int l = __ffs(hit) - 1;
+          hit &= hit - 1;
+          const int64_t k = base + l;
+          const double* qj = qnode + (int64_t)__shfl_sync(0xffffffffu, j_mine, l) * NE;
 #pragma unroll
-        for (int r = 0; r < BS; ++r) {
-          const double f = -w * dinv[i * BS + r];
+          for (int u = 0; u < EL; ++u)
 #pragma unroll
-          for (int c = 0; c < BS; ++c) {
-            const double av = A.at(k, r, c);
-            if (av == 0.0) continue;
-#pragma unroll
-            for (int t = 0; t < 6; ++t) s[r * 6 + t] += f * av * qj[c * 6 + t];
-          }
+            for (int c = 0; c < BS; ++c) {
+              const double av = A.at(k, r[u], c);
+              if (av != 0.0) s[u] = fma(f[u] * av, qj[c * 6 + t[u]], s[u]);
+            }
         }
       }
     }
     bool nz = false;
 #pragma unroll
-    for (int e = 0; e < BS * 6; ++e) {
-      pv[q * BS * 6 + e] = s[e];
-      nz = nz || s[e] != 0.0;
-    }
-    nzflag[q] = nz ? 1 : 0;
+    for (int u = 0; u < EL; ++u)
+      if (lane + 32 * u < NE) {
+        pv[q * NE + lane + 32 * u] = s[u];
+        nz = nz || s[u] != 0.0;
+      }
+    const bool any = __any_sync(0xffffffffu, nz);
+    if (lane == 0) nzflag[q] = any ? 1 : 0;
   }
 }
 
-// block-row index of every block
+// block-row index of every block (a warp per row)
 __global__ void ks_block_rows(int64_t n_rows, const int32_t* __restrict__ rp, int32_t* __restrict__ row) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rows; i += (int64_t)gridDim.x * blockDim.x)
-    for (int32_t k = rp[i]; k < rp[i + 1]; ++k) row[k] = (int32_t)i;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n_rows; i += nw)
+    for (int32_t k = rp[i] + (threadIdx.x & 31); k < rp[i + 1]; k += 32) row[k] = (int32_t)i;
 }
 
-// nonzero blocks per row
+// nonzero blocks per row (a warp per row)
 __global__ void ks_count_nz(int64_t n_rows, const int32_t* __restrict__ rp, const uint8_t* __restrict__ nzflag,
                             int32_t* __restrict__ cnt) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rows; i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t c = 0;
-    for (int32_t k = rp[i]; k < rp[i + 1]; ++k) c += nzflag[k];
-    cnt[i] = c;
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n_rows; i += nw) {
+    int c = 0;
+    for (int32_t k = rp[i] + lane; k < rp[i + 1]; k += 32) c += nzflag[k];
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) cnt[i] = c;
   }
 }
 
-// copy the nonzero blocks of each row, in order (thread per row)
+// copy the nonzero blocks of each row, in order (a warp per row, its lanes along the values)
 __global__ void ks_compact(int64_t n_rows, int bsz, const int32_t* __restrict__ rp_in, const int32_t* __restrict__ ci_in,
                            const double* __restrict__ v_in, const uint8_t* __restrict__ nzflag,
                            const int32_t* __restrict__ rp_out, int32_t* __restrict__ ci_out, double* __restrict__ v_out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rows; i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t o = rp_out[i];
-    for (int32_t k = rp_in[i]; k < rp_in[i + 1]; ++k) {
-      if (!nzflag[k]) continue;
-      ci_out[o] = ci_in[k];
-      for (int e = 0; e < bsz; ++e) v_out[(int64_t)o * bsz + e] = v_in[(int64_t)k * bsz + e];
-      ++o;
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n_rows; i += nw) {
+    int64_t o = rp_out[i];
+    const int32_t k1 = rp_in[i + 1];
+    for (int32_t base = rp_in[i]; base < k1; base += 32) {
+      const int32_t k = base + lane;
+      const bool keep = k < k1 && nzflag[k];
+      unsigned mask = __ballot_sync(0xffffffffu, keep);
+      if (keep) ci_out[o + __popc(mask & ((1u << lane) - 1))] = ci_in[k];
+      while (mask) {
+        const int64_t from = base + __ffs(mask) - 1;
+        mask &= mask - 1;
+        for (int e = lane; e < bsz; e += 32) v_out[o * bsz + e] = v_in[from * bsz + e];
+        ++o;
+      }
     }
   }
 }
@@ -361,60 +453,84 @@ __global__ void __launch_bounds__(kSymThreads) ks_gemm_pattern(DMat A, const int
   }
 }
 
-// thread per block of C: C(i, J) = sum over A(i,:) in order of A(i,k) B(k, J) (B's block found by
-// binary search in its sorted row); nzflag = the block is not all zero
+// C(i, J) = sum over A(i,:) in order of A(i,k) B(k, J); nzflag = the block is not all zero.  A warp per
+// block of C: a lane per block of A's row searches B's sorted row for J, 32 searches at a time;
+// the blocks found are multiplied in order, a lane per entry of C's block.  (A thread per block runs
+// the searches one after the other and reads every block of A and B by itself: 2.0 ms per
+// 6x6 product on the levels of a 42,000-node matrix against 1.6.)
 template <int AR, int AK, int BC>
-__global__ void ks_gemm_values(DMat A, const int32_t* __restrict__ brp, const int32_t* __restrict__ bci,
-                               const double* __restrict__ bv, const int32_t* __restrict__ crow,
-                               const int32_t* __restrict__ cci, int64_t nnz, double* __restrict__ cv,
-                               uint8_t* __restrict__ nzflag) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nnz; q += (int64_t)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(kT) ks_gemm_values(DMat A, const int32_t* __restrict__ brp,
+                                                     const int32_t* __restrict__ bci, const double* __restrict__ bv,
+                                                     const int32_t* __restrict__ crow,
+                                                     const int32_t* __restrict__ cci, int64_t nnz,
+                                                     double* __restrict__ cv, uint8_t* __restrict__ nzflag) {
+  constexpr int NE = AR * BC, EL = (NE + 31) / 32;
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  int r[EL], t[EL];
+#pragma unroll
+  for (int u = 0; u < EL; ++u) {
+    const int e = min(lane + 32 * u, NE - 1);
+    r[u] = e / BC;
+    t[u] = e % BC;
+  }
+  for (int64_t q = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; q < nnz; q += nw) {
     const int64_t i = crow[q];
-    const int32_t J = cci[q];
-    double acc[AR * BC];
+    const int32_t J = cci[q], k1 = A.rp[i + 1];
+    double acc[EL] = {};
+    for (int32_t base = A.rp[i]; base < k1; base += 32) {
+      int32_t p_mine = -1;
+      if (base + lane < k1) {
+        const int32_t j = A.ci[base + lane];
+        p_mine = find_col(bci, brp[j], brp[j + 1], J);
+      }
+      unsigned hit = __ballot_sync(0xffffffffu, p_mine >= 0);
+      while (hit) {
+        const int l = __ffs(hit) - 1;
+        hit &= hit - 1;
+        const int64_t k = base + l;
+        const double* b = bv + (int64_t)__shfl_sync(0xffffffffu, p_mine, l) * AK * BC;
 #pragma unroll
-    for (int e = 0; e < AR * BC; ++e) acc[e] = 0.0;
-    for (int32_t k = A.rp[i]; k < A.rp[i + 1]; ++k) {
-      const int32_t j = A.ci[k];
-      const int32_t p = find_col(bci, brp[j], brp[j + 1], J);
-      if (p < 0) continue;
-      const double* b = bv + (int64_t)p * AK * BC;
+        for (int u = 0; u < EL; ++u)
 #pragma unroll
-      for (int r = 0; r < AR; ++r)
-#pragma unroll
-        for (int s = 0; s < AK; ++s) {
-          const double av = A.at(k, r, s);
-#pragma unroll
-          for (int t = 0; t < BC; ++t) acc[r * BC + t] += av * b[s * BC + t];
-        }
+          for (int m = 0; m < AK; ++m) acc[u] = fma(A.at(k, r[u], m), b[m * BC + t[u]], acc[u]);
+      }
     }
     bool nz = false;
 #pragma unroll
-    for (int e = 0; e < AR * BC; ++e) {
-      cv[q * AR * BC + e] = acc[e];
-      nz = nz || acc[e] != 0.0;
-    }
-    nzflag[q] = nz ? 1 : 0;
+    for (int u = 0; u < EL; ++u)
+      if (lane + 32 * u < NE) {
+        cv[q * NE + lane + 32 * u] = acc[u];
+        nz = nz || acc[u] != 0.0;
+      }
+    const bool any = __any_sync(0xffffffffu, nz);
+    if (lane == 0) nzflag[q] = any ? 1 : 0;
   }
 }
 
-// A <- (A + A^T) / 2 for a structurally symmetric block matrix (b x b blocks, thread per row)
-__global__ void ks_symmetrize(int64_t n_rows, int b, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                              const double* __restrict__ v, double* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rows; i += (int64_t)gridDim.x * blockDim.x)
-    for (int32_t k = rp[i]; k < rp[i + 1]; ++k) {
+// A <- (A + A^T) / 2 for a structurally symmetric block matrix (b x b blocks).  A warp per 32
+// blocks: each lane finds the mirror of its block, then the lanes go along the values of one block
+// after the other.
+__global__ void ks_symmetrize(int64_t nnz, int b, const int32_t* __restrict__ row, const int32_t* __restrict__ rp,
+                              const int32_t* __restrict__ ci, const double* __restrict__ v, double* __restrict__ out) {
+  const int lane = threadIdx.x & 31, nb = b * b;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t base = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; base < nnz; base += nw * 32) {
+    const int64_t k = base + lane;
+    int32_t f_mine = -1;
+    if (k < nnz) {
       const int32_t j = ci[k];
-      const int32_t f = find_col(ci, rp[j], rp[j + 1], (int32_t)i);
-      const double* x = v + (int64_t)k * b * b;
-      double* o = out + (int64_t)k * b * b;
-      if (f < 0) {
-        for (int e = 0; e < b * b; ++e) o[e] = x[e];
-        continue;
-      }
-      const double* y = v + (int64_t)f * b * b;
-      for (int r = 0; r < b; ++r)
-        for (int c = 0; c < b; ++c) o[r * b + c] = 0.5 * (x[r * b + c] + y[c * b + r]);
+      f_mine = find_col(ci, rp[j], rp[j + 1], row[k]);
     }
+    const int n = (int)min((int64_t)32, nnz - base);
+    for (int q = 0; q < n; ++q) {
+      const int32_t f = __shfl_sync(0xffffffffu, f_mine, q);
+      const double* x = v + (base + q) * nb;
+      double* o = out + (base + q) * nb;
+      const double* y = v + (int64_t)f * nb;
+      for (int e = lane; e < nb; e += 32) o[e] = f < 0 ? x[e] : 0.5 * (x[e] + y[e % b * b + e / b]);
+    }
+  }
 }
 
 __global__ void ks_to_float(int64_t n, const double* __restrict__ a, float* __restrict__ b) {
@@ -577,20 +693,27 @@ int scan_counts(const DArray<int32_t>& cnt, int64_t n, DArray<int32_t>& rp, std:
   return 0;
 }
 
-// drop all-zero blocks: (rp_t, ci_t, v_t, flags) -> M (rp, ci, v64 set; host row pointer too)
-int compact_into(int64_t n_rows, int br, int bc, int64_t n_cols, const DArray<int32_t>& rp_t,
-                 const DArray<int32_t>& ci_t, const DArray<double>& v_t, const DArray<uint8_t>& flags, DevBsr& M,
+// drop all-zero blocks: (rp_t, ci_t, v_t, flags) -> M (rp, ci, v64 set; host row pointer too); without one
+// (most products) the arrays themselves become M's
+int compact_into(int64_t n_rows, int br, int bc, int64_t n_cols, int64_t nnz_t, DArray<int32_t>& rp_t,
+                 DArray<int32_t>& ci_t, DArray<double>& v_t, const DArray<uint8_t>& flags, DevBsr& M,
                  std::vector<int32_t>& h_rp) {
   DArray<int32_t> cnt;
   WN_CHECK(cnt.alloc(std::max<int64_t>(n_rows, 1)));
-  ks_count_nz<<<grid_n(n_rows), kT>>>(n_rows, rp_t.p, flags.p, cnt.p);
+  ks_count_nz<<<grid_for(n_rows, 32, kT, 16), kT>>>(n_rows, rp_t.p, flags.p, cnt.p);
   WN_CUDA(cudaGetLastError());
   int64_t nnz = 0;
   WN_CHECK(scan_counts(cnt, n_rows, M.rp, h_rp, &nnz));
-  WN_CHECK(M.ci.alloc(std::max<int64_t>(nnz, 1)));
-  WN_CHECK(M.v64.alloc(std::max<int64_t>(nnz, 1) * br * bc));
-  ks_compact<<<grid_n(n_rows), kT>>>(n_rows, br * bc, rp_t.p, ci_t.p, v_t.p, flags.p, M.rp.p, M.ci.p, M.v64.p);
-  WN_CUDA(cudaGetLastError());
+  if (nnz == nnz_t && nnz > 0) {
+    M.ci = std::move(ci_t);
+    M.v64 = std::move(v_t);
+  } else {
+    WN_CHECK(M.ci.alloc(std::max<int64_t>(nnz, 1)));
+    WN_CHECK(M.v64.alloc(std::max<int64_t>(nnz, 1) * br * bc));
+    ks_compact<<<grid_for(n_rows, 32, kT, 16), kT>>>(n_rows, br * bc, rp_t.p, ci_t.p, v_t.p, flags.p, M.rp.p, M.ci.p,
+                                                     M.v64.p);
+    WN_CUDA(cudaGetLastError());
+  }
   M.br = br;
   M.bc = bc;
   M.n_rows = n_rows;
@@ -629,19 +752,49 @@ int power_rho_device(const DMat& A, const DArray<double>& dinv, int iters, doubl
   double* xp = x.p;
   double* yp = y.p;
   for (int it = 0; it < std::max(iters, 1); ++it) {
-    double nx = 0.0;
-    WN_CHECK(norm(xp, nullptr, &nx));
+    double nx = lam;  // x is the last step's scaled y, whose norm is known
+    if (it == 0) WN_CHECK(norm(xp, nullptr, &nx));
     if (nx == 0.0) {
       *rho = 1.0;
       return 0;
     }
     ks_divide<<<g, kT>>>(n, xp, nx);
-    ks_spmv_rows<<<grid_n(n), kT>>>(A, xp, yp);
+    if (A.br == 3)
+      ks_spmv_rows<3><<<grid_for(A.n_rows, 32, kT, 16), kT>>>(A, xp, yp);
+    else
+      ks_spmv_rows<6><<<grid_for(A.n_rows, 32, kT, 16), kT>>>(A, xp, yp);
     WN_CUDA(cudaGetLastError());
     WN_CHECK(norm(yp, dinv.p, &lam));
     std::swap(xp, yp);
   }
   *rho = lam;
+  return 0;
+}
+
+// The greedy aggregation (aggregate_norms) of a matrix with block norms nrm: strength and pass 2 on
+// the device, the sequential passes 1 and 3 on the host.
+int aggregate_device(const DMat& A, const DArray<double>& nrm, double theta, const int32_t* h_rp, const int32_t* h_ci,
+                     std::vector<int32_t>& agg, int64_t* n_agg) {
+  const int64_t n = A.n_rows, nnz = std::max<int64_t>(A.nnzb, 1);
+  DArray<double> dn;
+  DArray<uint8_t> strong, has;
+  DArray<int32_t> d_agg, d_out;
+  WN_CHECK(dn.alloc(n));
+  WN_CHECK(strong.alloc(nnz));
+  WN_CHECK(has.alloc(n));
+  ks_diag_norms<<<grid_n(n), kT>>>(n, A.rp, A.ci, nrm.p, dn.p);
+  ks_strong<<<grid_for(n, 32, kT, 16), kT>>>(n, A.rp, A.ci, nrm.p, dn.p, theta, strong.p, has.p);
+  WN_CUDA(cudaGetLastError());
+  std::vector<uint8_t> h_strong, h_has;
+  WN_CHECK(download(strong, A.nnzb, h_strong));
+  WN_CHECK(download(has, n, h_has));
+  int64_t na = aggregate_roots(n, h_rp, h_ci, h_strong.data(), h_has.data(), agg);
+  WN_CHECK(d_agg.upload(agg));
+  WN_CHECK(d_out.alloc(n));
+  ks_join<<<grid_n(n), kT>>>(n, A.rp, A.ci, nrm.p, strong.p, d_agg.p, d_out.p);
+  WN_CUDA(cudaGetLastError());
+  WN_CHECK(download(d_out, n, agg));
+  *n_agg = aggregate_leftovers(n, h_rp, h_ci, h_strong.data(), h_has.data(), na, agg);
   return 0;
 }
 
@@ -666,14 +819,14 @@ int gemm(const DMat& A, const DevBsr& B, DevBsr& C, std::vector<int32_t>& h_rp) 
   WN_CHECK(ci_t.alloc(std::max<int64_t>(nnz, 1)));
   WN_CHECK(row_t.alloc(std::max<int64_t>(nnz, 1)));
   ks_gemm_pattern<<<gs, kSymThreads>>>(A, B.rp.p, B.ci.p, nullptr, rp_t.p, ci_t.p, err.p);
-  ks_block_rows<<<grid_n(n), kT>>>(n, rp_t.p, row_t.p);
+  ks_block_rows<<<grid_for(n, 32, kT, 16), kT>>>(n, rp_t.p, row_t.p);
   DArray<double> v_t;
   DArray<uint8_t> flags;
   WN_CHECK(v_t.alloc(std::max<int64_t>(nnz, 1) * AR * BC));
   WN_CHECK(flags.alloc(std::max<int64_t>(nnz, 1)));
-  ks_gemm_values<AR, AK, BC><<<grid_n(nnz), kT>>>(A, B.rp.p, B.ci.p, B.v64.p, row_t.p, ci_t.p, nnz, v_t.p, flags.p);
+  ks_gemm_values<AR, AK, BC><<<grid_for(nnz, 32, kT, 16), kT>>>(A, B.rp.p, B.ci.p, B.v64.p, row_t.p, ci_t.p, nnz, v_t.p, flags.p);
   WN_CUDA(cudaGetLastError());
-  return compact_into(n, AR, BC, B.n_cols, rp_t, ci_t, v_t, flags, C, h_rp);
+  return compact_into(n, AR, BC, B.n_cols, nnz, rp_t, ci_t, v_t, flags, C, h_rp);
 }
 
 int gemm_any(const DMat& A, const DevBsr& B, DevBsr& C, std::vector<int32_t>& h_rp) {
@@ -696,7 +849,7 @@ int transpose(const DevBsr& M, DevBsr& T, std::vector<int32_t>& h_rp) {
   WN_CHECK(trow.alloc(std::max<int64_t>(nnz, 1)));
   WN_CHECK(tsrc.alloc(std::max<int64_t>(nnz, 1)));
   ks_col_count<<<grid_n(nnz), kT>>>(nnz, M.ci.p, cnt.p);
-  ks_block_rows<<<grid_n(M.n_rows), kT>>>(M.n_rows, M.rp.p, row.p);
+  ks_block_rows<<<grid_for(M.n_rows, 32, kT, 16), kT>>>(M.n_rows, M.rp.p, row.p);
   WN_CUDA(cudaGetLastError());
   int64_t total = 0;
   WN_CHECK(scan_counts(cnt, M.n_cols, T.rp, h_rp, &total));
@@ -735,7 +888,9 @@ int amg_build_device(Solid* s, const wn_amg_params& prm, AmgHierarchy& H) {
   // level 0: the assembled matrix in place (component-major 3x3, or row-major 6x6)
   DMat A{s->bs, s->bs, s->n_nodes, s->n_nodes, s->nnzb, s->row_ptr.p, s->col_idx.p, s->k64.p,
          s->bs == 3 ? s->nnzb : 0};
-  std::vector<int32_t> h_rp = s->h_row_ptr, h_ci = s->h_col_idx;
+  // host row pointers and columns of the current level's matrix
+  std::vector<int32_t> h_rp_own, h_ci_own;
+  const int32_t *h_rp = s->h_row_ptr.data(), *h_ci = s->h_col_idx.data();
   DevBsr A_own;  // the current level's matrix for levels >= 1
   int bs = s->bs;
   int64_t n = s->n_nodes;
@@ -760,10 +915,8 @@ int amg_build_device(Solid* s, const wn_amg_params& prm, AmgHierarchy& H) {
     WN_CHECK(nrm.alloc(std::max<int64_t>(A.nnzb, 1)));
     ks_block_norms<<<grid_n(A.nnzb), kT>>>(A, nrm.p);
     WN_CUDA(cudaGetLastError());
-    std::vector<double> h_nrm;
-    WN_CHECK(download(nrm, A.nnzb, h_nrm));
+    WN_CHECK(aggregate_device(A, nrm, prm.strength_theta, h_rp, h_ci, L.agg, &L.n_agg));
     nrm.release();
-    L.n_agg = aggregate_norms(n, h_rp.data(), h_ci.data(), h_nrm.data(), prm.strength_theta, L.agg);
     if (L.n_agg == 0 || L.n_agg * 6 >= (int64_t)(0.8 * ndof)) break;  // coarsening stalled
     std::vector<double> Qnode, Bc;
     tentative_prolongator(n, bs, L.n_agg, L.agg, B, Qnode, Bc);
@@ -794,14 +947,14 @@ int amg_build_device(Solid* s, const wn_amg_params& prm, AmgHierarchy& H) {
     WN_CHECK(v_t.alloc(std::max<int64_t>(nnz_t, 1) * bs * 6));
     WN_CHECK(flags.alloc(std::max<int64_t>(nnz_t, 1)));
     ks_p_pattern<<<gw, kT>>>(A, d_agg.p, smooth, nullptr, rp_t.p, ci_t.p, err.p);
-    ks_block_rows<<<grid_n(n), kT>>>(n, rp_t.p, row_t.p);
+    ks_block_rows<<<grid_for(n, 32, kT, 16), kT>>>(n, rp_t.p, row_t.p);
     if (bs == 3)
-      ks_p_values<3><<<grid_n(nnz_t), kT>>>(A, d_agg.p, d_q.p, D.dinv64.p, w, row_t.p, ci_t.p, nnz_t, v_t.p, flags.p);
+      ks_p_values<3><<<grid_for(nnz_t, 32, kT, 16), kT>>>(A, d_agg.p, d_q.p, D.dinv64.p, w, row_t.p, ci_t.p, nnz_t, v_t.p, flags.p);
     else
-      ks_p_values<6><<<grid_n(nnz_t), kT>>>(A, d_agg.p, d_q.p, D.dinv64.p, w, row_t.p, ci_t.p, nnz_t, v_t.p, flags.p);
+      ks_p_values<6><<<grid_for(nnz_t, 32, kT, 16), kT>>>(A, d_agg.p, d_q.p, D.dinv64.p, w, row_t.p, ci_t.p, nnz_t, v_t.p, flags.p);
     WN_CUDA(cudaGetLastError());
     std::vector<int32_t> h_rp_p, h_rp_r, h_rp_ap, h_rp_c;
-    WN_CHECK(compact_into(n, bs, 6, L.n_agg, rp_t, ci_t, v_t, flags, D.P, h_rp_p));
+    WN_CHECK(compact_into(n, bs, 6, L.n_agg, nnz_t, rp_t, ci_t, v_t, flags, D.P, h_rp_p));
     rp_t.release();
     ci_t.release();
     row_t.release();
@@ -821,7 +974,9 @@ int amg_build_device(Solid* s, const wn_amg_params& prm, AmgHierarchy& H) {
     AP = DevBsr();
     DArray<double> sym;
     WN_CHECK(sym.alloc(std::max<int64_t>(Ac.nnzb, 1) * 36));
-    ks_symmetrize<<<grid_n(Ac.n_rows), kT>>>(Ac.n_rows, 6, Ac.rp.p, Ac.ci.p, Ac.v64.p, sym.p);
+    WN_CHECK(row_t.alloc(std::max<int64_t>(Ac.nnzb, 1)));
+    ks_block_rows<<<grid_for(Ac.n_rows, 32, kT, 16), kT>>>(Ac.n_rows, Ac.rp.p, row_t.p);
+    ks_symmetrize<<<grid_n(Ac.nnzb), kT>>>(Ac.nnzb, 6, row_t.p, Ac.rp.p, Ac.ci.p, Ac.v64.p, sym.p);
     WN_CUDA(cudaGetLastError());
     std::swap(Ac.v64, sym);
     tr.mark("R*(AP)", lvl);
@@ -830,14 +985,16 @@ int amg_build_device(Solid* s, const wn_amg_params& prm, AmgHierarchy& H) {
     D.h_R_rp = std::move(h_rp_r);
     if (lvl > 0) {
       D.A = std::move(A_own);
-      D.h_A_rp = h_rp;
+      D.h_A_rp = h_rp_own;
     }
     host.levels.push_back(std::move(L));
     H.levels.push_back(std::move(D));
     A_own = std::move(Ac);
     A = dmat(A_own);
-    h_rp = std::move(h_rp_c);
-    WN_CHECK(download(A_own.ci, A_own.nnzb, h_ci));
+    h_rp_own = std::move(h_rp_c);
+    WN_CHECK(download(A_own.ci, A_own.nnzb, h_ci_own));
+    h_rp = h_rp_own.data();
+    h_ci = h_ci_own.data();
     B.swap(Bc);
     bs = 6;
     n = host.levels.back().n_agg;
@@ -855,12 +1012,10 @@ int amg_build_device(Solid* s, const wn_amg_params& prm, AmgHierarchy& H) {
       } else {
         v.swap(raw);
       }
-      h_rp = s->h_row_ptr;
-      h_ci = s->h_col_idx;
     } else {
       WN_CHECK(download(A_own.v64, A.nnzb * bs * bs, v));
     }
-    WN_CHECK(dense_coarse(n, bs, h_rp.data(), h_ci.data(), v.data(), host));
+    WN_CHECK(dense_coarse(n, bs, h_rp, h_ci, v.data(), host));
     tr.mark("coarse", -1);
   }
   // FP32 copies
@@ -896,7 +1051,7 @@ int amg_coarse_block_basis(AmgHierarchy& H, const wn_amg_params& prm) {
   }
   auto rows_of = [&](const DevBsr& M, DArray<int32_t>& row) -> int {
     WN_CHECK(row.alloc(std::max<int64_t>(M.nnzb, 1)));
-    ks_block_rows<<<grid_n(M.n_rows), kT>>>(M.n_rows, M.rp.p, row.p);
+    ks_block_rows<<<grid_for(M.n_rows, 32, kT, 16), kT>>>(M.n_rows, M.rp.p, row.p);
     WN_CUDA(cudaGetLastError());
     return 0;
   };

@@ -390,6 +390,38 @@ void symmetrize(HostBsr& A) {
 
 }  // namespace
 
+// pass 1 of the aggregation: roots whose strong neighbourhood is free; their number
+int64_t aggregate_roots(int64_t n, const int32_t* rp, const int32_t* ci, const uint8_t* strong,
+                        const uint8_t* has_strong, std::vector<int32_t>& agg) {
+  agg.assign(n, -1);
+  int64_t na = 0;
+  for (int64_t i = 0; i < n; ++i) {
+    if (agg[i] >= 0 || !has_strong[i]) continue;
+    bool free_all = true;
+    for (int32_t k = rp[i]; k < rp[i + 1] && free_all; ++k)
+      if (strong[k] && agg[ci[k]] >= 0) free_all = false;
+    if (!free_all) continue;
+    agg[i] = (int32_t)na;
+    for (int32_t k = rp[i]; k < rp[i + 1]; ++k)
+      if (strong[k]) agg[ci[k]] = (int32_t)na;
+    ++na;
+  }
+  return na;
+}
+
+// pass 3: leftovers with strong links form new aggregates after the first na; the number of all
+int64_t aggregate_leftovers(int64_t n, const int32_t* rp, const int32_t* ci, const uint8_t* strong,
+                            const uint8_t* has_strong, int64_t na, std::vector<int32_t>& agg) {
+  for (int64_t i = 0; i < n; ++i) {
+    if (agg[i] >= 0 || !has_strong[i]) continue;
+    agg[i] = (int32_t)na;
+    for (int32_t k = rp[i]; k < rp[i + 1]; ++k)
+      if (strong[k] && agg[ci[k]] < 0) agg[ci[k]] = (int32_t)na;
+    ++na;
+  }
+  return na;
+}
+
 // Three-pass greedy aggregation (Vanek-Mandel-Brezina) on the strong block graph, given the
 // Frobenius norm of every block: (i, j) is strong if |A_ij| >= theta sqrt(|A_ii| |A_jj|).
 // Pass 1 makes roots of nodes whose strong neighbourhood is still free; pass 2 joins each left
@@ -413,19 +445,7 @@ int64_t aggregate_norms(int64_t n, const int32_t* rp, const int32_t* ci, const d
         }
       }
   });
-  agg.assign(n, -1);
-  int64_t na = 0;
-  for (int64_t i = 0; i < n; ++i) {  // pass 1: roots whose strong neighbourhood is free
-    if (agg[i] >= 0 || !has_strong[i]) continue;
-    bool free_all = true;
-    for (int32_t k = rp[i]; k < rp[i + 1] && free_all; ++k)
-      if (strong[k] && agg[ci[k]] >= 0) free_all = false;
-    if (!free_all) continue;
-    agg[i] = (int32_t)na;
-    for (int32_t k = rp[i]; k < rp[i + 1]; ++k)
-      if (strong[k]) agg[ci[k]] = (int32_t)na;
-    ++na;
-  }
+  const int64_t na = aggregate_roots(n, rp, ci, strong.data(), has_strong.data(), agg);
   std::vector<int32_t> pass2(agg);
   for (int64_t i = 0; i < n; ++i) {  // pass 2: join the strongest aggregated neighbour
     if (agg[i] >= 0 || !has_strong[i]) continue;
@@ -439,14 +459,7 @@ int64_t aggregate_norms(int64_t n, const int32_t* rp, const int32_t* ci, const d
     pass2[i] = ba;
   }
   agg.swap(pass2);
-  for (int64_t i = 0; i < n; ++i) {  // pass 3: leftovers with strong links form new aggregates
-    if (agg[i] >= 0 || !has_strong[i]) continue;
-    agg[i] = (int32_t)na;
-    for (int32_t k = rp[i]; k < rp[i + 1]; ++k)
-      if (strong[k] && agg[ci[k]] < 0) agg[ci[k]] = (int32_t)na;
-    ++na;
-  }
-  return na;
+  return aggregate_leftovers(n, rp, ci, strong.data(), has_strong.data(), na, agg);
 }
 
 // Near-null space of level 0: the 6 rigid-body modes, zero on fixed DOFs.  Rows ux, uy, uz (and

@@ -47,6 +47,10 @@ wn_amg_params amg_default_params();
 // greedy aggregation from block norms (-1 = unaggregated); the rigid-body near-null space of
 // level 0; the tentative prolongator (per-aggregate QR: Qnode n x bs x 6, Bc n_agg x 36); the
 // dense coarsest level (out.n_coarse, coarse_A, coarse_inv).
+int64_t aggregate_roots(int64_t n, const int32_t* rp, const int32_t* ci, const uint8_t* strong,
+                        const uint8_t* has_strong, std::vector<int32_t>& agg);
+int64_t aggregate_leftovers(int64_t n, const int32_t* rp, const int32_t* ci, const uint8_t* strong,
+                            const uint8_t* has_strong, int64_t na, std::vector<int32_t>& agg);
 int64_t aggregate_norms(int64_t n, const int32_t* rp, const int32_t* ci, const double* nrm, double theta,
                         std::vector<int32_t>& agg);
 void near_null_space(int64_t n0, int bs0, const double* coords, const uint8_t* fixed, std::vector<double>& B);
