@@ -28,6 +28,11 @@ constexpr int KE_TILE = 16;      // elements per CTA
 constexpr int KE_THREADS = 256;  // threads per CTA
 
 // Stage one element's coordinates: X[a][j] = nodes[conn[e][a]][j].
+__device__ __forceinline__ void cp_async4(int32_t* smem, const int32_t* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(gmem) : "memory");
+}
+
 __device__ __forceinline__ void load_coords(const double* __restrict__ nodes, const int32_t* __restrict__ conn,
                                             int64_t e, double X[10][3]) {
 #pragma unroll
@@ -472,71 +477,215 @@ __global__ void __launch_bounds__(kAsmThreads, 2) assemble_tiles_kernel(
   }
 }
 
+// Element passes over a displacement field (forces, energies, stresses), a thread per element.
+//
+// The shape functions are quadratic in the volume coordinates L, so a gradient dx/dL_j is linear and
+// its value at Gauss point g is alpha sum_v D_j(v) + (beta - alpha) D_j(g), from its values at the
+// four vertices:  D_j(v) = 4 x_(v,j) - x_j  (x_(v,j): the node amid edge v-j),  D_v(v) = 3 x_v.
+// Coordinates and displacements need 7 nodes per point that way, in differences from node g, where the
+// derivatives of all ten shape functions were formed at each point and summed over; the nodal forces
+// are the transposed sums.  Instructions per element: forces 2,336 -> 1,670, stresses 1,844 -> 1,185.
+// An element's 60 values stay in registers (250 of them, 8 warps per SM): in shared memory, at 12
+// warps, the kernels were bound by its wavefronts (37 and 34 us where these take 28 and 22).
+constexpr int kElWarps = 4;   // per block; each warp takes runs of 32 elements by itself
+constexpr int kElPitch = 33;  // of one component's values; odd, so that rows and columns are both free of conflicts
+
+__host__ __device__ constexpr int edge_node(int i, int j) {
+  const int lo = i < j ? i : j, hi = i < j ? j : i;
+  return lo == 0 ? (hi == 1 ? 4 : hi == 2 ? 6 : 7) : lo == 1 ? (hi == 2 ? 5 : 8) : 9;
+}
+
+// sum over the vertices of D_k - D_0 (k = 1, 2, 3): 4 (the nodes amid k's edges - those amid 0's)
+__device__ __forceinline__ void el_vertex_sum(const double X[10][3], double S[3][3]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double e01 = X[4][c], e12 = X[5][c], e02 = X[6][c], e03 = X[7][c],
+                 e13 = X[8][c], e23 = X[9][c];
+    S[0][c] = 4.0 * ((e12 - e02) + (e13 - e03));
+    S[1][c] = 4.0 * ((e12 - e01) + (e23 - e03));
+    S[2][c] = 4.0 * ((e13 - e01) + (e23 - e02));
+  }
+}
+
+// d/dL_k - d/dL_0 at Gauss point V, from the values relative to node V
+template <int V>
+__device__ __forceinline__ void el_gradient(const double X[10][3], const double S[3][3], double J[3][3]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double o = X[V][c];
+    double D[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      D[j] = j == V ? 0.0 : fma(4.0, X[edge_node(V, j)][c] - o, -(X[j][c] - o));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) J[k][c] = fma(kBeta - kAlpha, D[k + 1] - D[0], kAlpha * S[k][c]);
+  }
+}
+
+// det J and its inverse: inv[i][k] = dL_k/dx_i for J[k][j] = dx_j/dL_k
+__device__ __forceinline__ double el_inverse(const double J[3][3], double inv[3][3]) {
+  const double c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+  const double c01 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+  const double c02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+  const double det = J[0][0] * c00 + J[0][1] * c01 + J[0][2] * c02;
+  const double id = 1.0 / det;
+  inv[0][0] = c00 * id;
+  inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
+  inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
+  inv[1][0] = c01 * id;
+  inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
+  inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * id;
+  inv[2][0] = c02 * id;
+  inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * id;
+  inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
+  return det;
+}
+
+// stress [sxx, syy, szz, sxy, syz, szx] at Gauss point V; inv and det of its Jacobian on return
+template <int V>
+__device__ __forceinline__ double el_stress(const double X[10][3], const double u[10][3], const double SX[3][3],
+                                            const double SU[3][3], double c11, double c12, double G,
+                                            double inv[3][3], double s[6]) {
+  double J[3][3];
+  el_gradient<V>(X, SX, J);
+  const double det = el_inverse(J, inv);
+  double U[3][3], H[3][3];  // du_c/dL_k, du_c/dx_i
+  el_gradient<V>(u, SU, U);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) H[i][c] = fma(inv[i][0], U[0][c], fma(inv[i][1], U[1][c], inv[i][2] * U[2][c]));
+  s[0] = c11 * H[0][0] + c12 * H[1][1] + c12 * H[2][2];
+  s[1] = c12 * H[0][0] + c11 * H[1][1] + c12 * H[2][2];
+  s[2] = c12 * H[0][0] + c12 * H[1][1] + c11 * H[2][2];
+  s[3] = G * (H[1][0] + H[0][1]);
+  s[4] = G * (H[2][1] + H[1][2]);
+  s[5] = G * (H[2][0] + H[0][2]);
+  return det;
+}
+
+// connectivity of elements e0 .. e0 + 31 on its way to shared memory
+__device__ __forceinline__ void el_fetch(int32_t* s_conn, const int32_t* __restrict__ conn, int64_t e0, int64_t n_el,
+                                         int lane) {
+  if (e0 < n_el) {
+    const int n = (int)(n_el - e0 < 32 ? n_el - e0 : 32) * 10;
+#pragma unroll
+    for (int j = 0; j < 10; ++j)
+      if (j * 32 + lane < n) cp_async4(s_conn + j * 32 + lane, conn + e0 * 10 + j * 32 + lane);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// the coordinates and displacements of the ten nodes of the thread's element
+__device__ __forceinline__ void el_load(const double* __restrict__ nodes, const int32_t* s_conn,
+                                        const double* __restrict__ u, int stride, double X[10][3], double ue[10][3]) {
+  int2 n[5];
+#pragma unroll
+  for (int a = 0; a < 5; ++a) n[a] = reinterpret_cast<const int2*>(s_conn)[a];
+#pragma unroll
+  for (int a = 0; a < 10; ++a) {
+    const int64_t v = a & 1 ? n[a / 2].y : n[a / 2].x;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      X[a][c] = nodes[v * 3 + c];
+      ue[a][c] = u[v * stride + c];
+    }
+  }
+}
+
+// contribution of Gauss point V to P[v][k][c], the derivative of the energy by D_k(v) of component c
+template <int V>
+__device__ __forceinline__ bool el_force_point(const double X[10][3], const double u[10][3], const double SX[3][3],
+                                               const double SU[3][3], double c11, double c12, double G,
+                                               double P[3][3]) {
+  double inv[3][3], s[6];
+  const double det = el_stress<V>(X, u, SX, SU, c11, c12, G, inv, s);
+  const double w = kWeight * det;
+  const double t[3][3] = {{w * s[0], w * s[3], w * s[5]}, {w * s[3], w * s[1], w * s[4]}, {w * s[5], w * s[4], w * s[2]}};
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) P[k][c] = fma(t[c][0], inv[0][k], fma(t[c][1], inv[1][k], t[c][2] * inv[2][k]));
+  return det > 0.0;
+}
+
 // Matrix-free element forces f_e = Ke u_e (= sum_g w|J| B^T C B u_e, c3d10.py:252-283) for
 // DOF stride `stride` (3 for the solid path, 6 for the reference's mixed-DOF layout of
 // kernels.cpp:244-376).  If fe_out: writes f_e (n_el x 30).  If energy_out: writes
 // u_e . f_e per element.  If grad_e: writes -u_e . f_e / E_e (compliance adjoint).
-__global__ void element_force_kernel(int64_t n_el, const double* __restrict__ nodes, const int32_t* __restrict__ conn,
-                                     const double* __restrict__ props, const double* __restrict__ u, int stride,
-                                     double* __restrict__ fe_out, double* __restrict__ energy_out,
-                                     double* __restrict__ grad_e, int* __restrict__ flags) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_el; e += (int64_t)gridDim.x * blockDim.x) {
-    double X[10][3], ue[10][3];
-    load_coords(nodes, conn, e, X);
-#pragma unroll
-    for (int a = 0; a < 10; ++a) {
-      const int64_t n = conn[e * 10 + a];
-      ue[a][0] = u[n * stride + 0];
-      ue[a][1] = u[n * stride + 1];
-      ue[a][2] = u[n * stride + 2];
-    }
-    const double E = props[e * 2], nu = props[e * 2 + 1];
-    const double f = E / ((1.0 + nu) * (1.0 - 2.0 * nu));
-    const double c11 = f * (1.0 - nu), c12 = f * nu, G = E / (2.0 * (1.0 + nu));
-    double fe[10][3];
-#pragma unroll
-    for (int a = 0; a < 10; ++a) fe[a][0] = fe[a][1] = fe[a][2] = 0.0;
-    bool bad = false;
-#pragma unroll 1
-    for (int g = 0; g < 4; ++g) {
-      double d[3][10];
-      const double det = gp_cartesian(g, X, d);
-      if (!(det > 0.0)) bad = true;
-      double eps[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-      for (int a = 0; a < 10; ++a) {
-        eps[0] += d[0][a] * ue[a][0];
-        eps[1] += d[1][a] * ue[a][1];
-        eps[2] += d[2][a] * ue[a][2];
-        eps[3] += d[1][a] * ue[a][0] + d[0][a] * ue[a][1];
-        eps[4] += d[2][a] * ue[a][1] + d[1][a] * ue[a][2];
-        eps[5] += d[2][a] * ue[a][0] + d[0][a] * ue[a][2];
+//
+// The next run's connectivity is fetched during this one's arithmetic, and the forces leave through
+// shared memory, so that consecutive lanes write consecutive values: a store of one component
+// from 32 elements touched 32 sectors and took 18 wavefronts.
+// Bound by latency at 8 warps per SM (FP64 pipe 46 %, L1 wavefronts 49 %): 61 -> 28 us for the forces of
+// 200,000 elements.
+__global__ void __launch_bounds__(kElWarps * 32, 2) element_force_kernel(
+    int64_t n_el, const double* __restrict__ nodes, const int32_t* __restrict__ conn, const double* __restrict__ props,
+    const double* __restrict__ u, int stride, double* __restrict__ fe_out, double* __restrict__ energy_out,
+    double* __restrict__ grad_e, int* __restrict__ flags) {
+  __shared__ __align__(16) int32_t s_conn[kElWarps][2][320];
+  __shared__ double s_fe[kElWarps][30 * kElPitch];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t step = (int64_t)gridDim.x * kElWarps * 32;
+  int64_t e0 = ((int64_t)blockIdx.x * kElWarps + warp) * 32;
+  el_fetch(s_conn[warp][0], conn, e0, n_el, lane);
+  for (int buf = 0; e0 < n_el; e0 += step, buf ^= 1) {
+    el_fetch(s_conn[warp][buf ^ 1], conn, e0 + step, n_el, lane);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const int64_t e = e0 + lane;
+    if (e < n_el) {
+      double X[10][3], ue[10][3];
+      el_load(nodes, s_conn[warp][buf] + lane * 10, u, stride, X, ue);
+      const double E = props[e * 2], nu = props[e * 2 + 1];
+      const double f = E / ((1.0 + nu) * (1.0 - 2.0 * nu));
+      const double c11 = f * (1.0 - nu), c12 = f * nu, G = E / (2.0 * (1.0 + nu));
+      double P[4][3][3];
+      bool good;
+      {
+        double SX[3][3], SU[3][3];
+        el_vertex_sum(X, SX);
+        el_vertex_sum(ue, SU);
+        good = el_force_point<0>(X, ue, SX, SU, c11, c12, G, P[0]);
+        good &= el_force_point<1>(X, ue, SX, SU, c11, c12, G, P[1]);
+        good &= el_force_point<2>(X, ue, SX, SU, c11, c12, G, P[2]);
+        good &= el_force_point<3>(X, ue, SX, SU, c11, c12, G, P[3]);
       }
-      const double s0 = c11 * eps[0] + c12 * eps[1] + c12 * eps[2];
-      const double s1 = c12 * eps[0] + c11 * eps[1] + c12 * eps[2];
-      const double s2 = c12 * eps[0] + c12 * eps[1] + c11 * eps[2];
-      const double s3 = G * eps[3], s4 = G * eps[4], s5 = G * eps[5];
-      const double w = kWeight * det;
-#pragma unroll
-      for (int a = 0; a < 10; ++a) {
-        fe[a][0] += w * (d[0][a] * s0 + d[1][a] * s3 + d[2][a] * s5);
-        fe[a][1] += w * (d[1][a] * s1 + d[0][a] * s3 + d[2][a] * s4);
-        fe[a][2] += w * (d[2][a] * s2 + d[1][a] * s4 + d[0][a] * s5);
-      }
-    }
-    if (bad) flags[0] = 1;
-    if (fe_out) {
-#pragma unroll
-      for (int a = 0; a < 10; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) fe_out[e * 30 + a * 3 + c] = fe[a][c];
-    }
-    if (energy_out || grad_e) {
+      if (!good) flags[0] = 1;
       double en = 0.0;
 #pragma unroll
-      for (int a = 0; a < 10; ++a) en += ue[a][0] * fe[a][0] + ue[a][1] * fe[a][1] + ue[a][2] * fe[a][2];
+      for (int c = 0; c < 3; ++c) {
+        double T[4], Q[4][4];  // by D_j of component c: sum over the points, at vertex v
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          T[k + 1] = (P[0][k][c] + P[1][k][c]) + (P[2][k][c] + P[3][k][c]);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) Q[v][k + 1] = fma(kBeta - kAlpha, P[v][k][c], kAlpha * T[k + 1]);
+        }
+        T[0] = -(T[1] + T[2] + T[3]);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) Q[v][0] = -(Q[v][1] + Q[v][2] + Q[v][3]);
+        double fe[10];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          fe[i] = fma(4.0, Q[i][i], -T[i]);
+#pragma unroll
+          for (int j = i + 1; j < 4; ++j) fe[edge_node(i, j)] = 4.0 * (Q[j][i] + Q[i][j]);
+        }
+#pragma unroll
+        for (int a = 0; a < 10; ++a) {
+          en = fma(ue[a][c], fe[a], en);
+          if (fe_out) s_fe[warp][(a * 3 + c) * kElPitch + lane] = fe[a];
+        }
+      }
       if (energy_out) energy_out[e] = en;
       if (grad_e) grad_e[e] = -en / E;
+    }
+    __syncwarp();
+    if (fe_out) {
+      const int n = (int)(n_el - e0 < 32 ? n_el - e0 : 32) * 30;
+      for (int i = lane; i < n; i += 32) fe_out[e0 * 30 + i] = s_fe[warp][(i % 30) * kElPitch + i / 30];
+      __syncwarp();
     }
   }
 }
@@ -563,57 +712,60 @@ __global__ void node_gather_kernel(int64_t n_nodes, const int64_t* __restrict__ 
 // mean Gauss-point von Mises (solid_solver.py:341-350, c3d10.py:286-318).
 // Also, when gp_sig / gp_vm are given, the stresses and von Mises of every Gauss point
 // (element_stresses_c3d10, c3d10.py:286-318): gp_sig[(e * 4 + g) * 6 + k], gp_vm[e * 4 + g].
-__global__ void stress_kernel(int64_t n_el, const double* __restrict__ nodes, const int32_t* __restrict__ conn,
-                              const double* __restrict__ props, const double* __restrict__ u,
-                              double* __restrict__ cell_sig, double* __restrict__ cell_vm, double* __restrict__ gp_sig,
-                              double* __restrict__ gp_vm) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_el; e += (int64_t)gridDim.x * blockDim.x) {
-    double X[10][3], ue[10][3];
-    load_coords(nodes, conn, e, X);
+// 32 -> 22 us for the 200,000 elements (FP64 pipe half busy).
+__global__ void __launch_bounds__(kElWarps * 32, 2) stress_kernel(
+    int64_t n_el, const double* __restrict__ nodes, const int32_t* __restrict__ conn, const double* __restrict__ props,
+    const double* __restrict__ u, double* __restrict__ cell_sig, double* __restrict__ cell_vm,
+    double* __restrict__ gp_sig, double* __restrict__ gp_vm) {
+  __shared__ __align__(16) int32_t s_conn[kElWarps][2][320];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t step = (int64_t)gridDim.x * kElWarps * 32;
+  int64_t e0 = ((int64_t)blockIdx.x * kElWarps + warp) * 32;
+  el_fetch(s_conn[warp][0], conn, e0, n_el, lane);
+  for (int buf = 0; e0 < n_el; e0 += step, buf ^= 1) {
+    el_fetch(s_conn[warp][buf ^ 1], conn, e0 + step, n_el, lane);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const int64_t e = e0 + lane;
+    if (e < n_el) {
+      double X[10][3], ue[10][3], SX[3][3], SU[3][3];
+      el_load(nodes, s_conn[warp][buf] + lane * 10, u, 3, X, ue);
+      const double E = props[e * 2], nu = props[e * 2 + 1];
+      const double f = E / ((1.0 + nu) * (1.0 - 2.0 * nu));
+      const double c11 = f * (1.0 - nu), c12 = f * nu, G = E / (2.0 * (1.0 + nu));
+      el_vertex_sum(X, SX);
+      el_vertex_sum(ue, SU);
+      double ssum[6] = {0, 0, 0, 0, 0, 0};
+      double vmsum = 0.0;
+      auto point = [&](int g, const double s[6]) {
 #pragma unroll
-    for (int a = 0; a < 10; ++a) {
-      const int64_t n = conn[e * 10 + a];
-      ue[a][0] = u[n * 3 + 0];
-      ue[a][1] = u[n * 3 + 1];
-      ue[a][2] = u[n * 3 + 2];
-    }
-    const double E = props[e * 2], nu = props[e * 2 + 1];
-    const double f = E / ((1.0 + nu) * (1.0 - 2.0 * nu));
-    const double c11 = f * (1.0 - nu), c12 = f * nu, G = E / (2.0 * (1.0 + nu));
-    double ssum[6] = {0, 0, 0, 0, 0, 0};
-    double vmsum = 0.0;
-#pragma unroll 1
-    for (int g = 0; g < 4; ++g) {
-      double d[3][10];
-      gp_cartesian(g, X, d);
-      double eps[6] = {0, 0, 0, 0, 0, 0};
+        for (int k = 0; k < 6; ++k) ssum[k] += s[k];
+        const double a0 = s[0] - s[1], a1 = s[1] - s[2], a2 = s[2] - s[0];
+        const double vm =
+            sqrt(0.5 * (a0 * a0 + a1 * a1 + a2 * a2 + 6.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5])));
+        vmsum += vm;
+        if (gp_sig) {
 #pragma unroll
-      for (int a = 0; a < 10; ++a) {
-        eps[0] += d[0][a] * ue[a][0];
-        eps[1] += d[1][a] * ue[a][1];
-        eps[2] += d[2][a] * ue[a][2];
-        eps[3] += d[1][a] * ue[a][0] + d[0][a] * ue[a][1];
-        eps[4] += d[2][a] * ue[a][1] + d[1][a] * ue[a][2];
-        eps[5] += d[2][a] * ue[a][0] + d[0][a] * ue[a][2];
+          for (int k = 0; k < 6; ++k) gp_sig[(e * 4 + g) * 6 + k] = s[k];
+          gp_vm[e * 4 + g] = vm;
+        }
+      };
+      double inv[3][3], s[6];
+      el_stress<0>(X, ue, SX, SU, c11, c12, G, inv, s);
+      point(0, s);
+      el_stress<1>(X, ue, SX, SU, c11, c12, G, inv, s);
+      point(1, s);
+      el_stress<2>(X, ue, SX, SU, c11, c12, G, inv, s);
+      point(2, s);
+      el_stress<3>(X, ue, SX, SU, c11, c12, G, inv, s);
+      point(3, s);
+      if (cell_sig) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) cell_sig[e * 6 + k] = ssum[k] / 4.0;
+        cell_vm[e] = vmsum / 4.0;
       }
-      const double s[6] = {c11 * eps[0] + c12 * eps[1] + c12 * eps[2], c12 * eps[0] + c11 * eps[1] + c12 * eps[2],
-                           c12 * eps[0] + c12 * eps[1] + c11 * eps[2], G * eps[3], G * eps[4], G * eps[5]};
-#pragma unroll
-      for (int k = 0; k < 6; ++k) ssum[k] += s[k];
-      const double a0 = s[0] - s[1], a1 = s[1] - s[2], a2 = s[2] - s[0];
-      const double vm = sqrt(0.5 * (a0 * a0 + a1 * a1 + a2 * a2 + 6.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5])));
-      vmsum += vm;
-      if (gp_sig) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) gp_sig[(e * 4 + g) * 6 + k] = s[k];
-        gp_vm[e * 4 + g] = vm;
-      }
     }
-    if (cell_sig) {
-#pragma unroll
-      for (int k = 0; k < 6; ++k) cell_sig[e * 6 + k] = ssum[k] / 4.0;
-      cell_vm[e] = vmsum / 4.0;
-    }
+    __syncwarp();
   }
 }
 
@@ -632,6 +784,11 @@ __global__ void nodal_average_kernel(int64_t n_nodes, const int64_t* __restrict_
 // ---------------------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------------------
+// one wave: two blocks per SM by their registers
+int el_grid(int64_t n_el) {
+  return (int)std::min<int64_t>((n_el + kElWarps * 32 - 1) / (kElWarps * 32), (int64_t)kNumSMs * 2);
+}
+
 size_t assemble_tiles_smem(int ne_max, int max_codes) {
   return (size_t)(asm_el_area(ne_max) + asm_union_doubles(ne_max)) * sizeof(double) +
          ((size_t)max_codes * 2 + 7) / 8 * 8;
@@ -808,8 +965,7 @@ int launch_element_force(int64_t n_el, const double* nodes, const int32_t* conn,
                          const double* u, int stride, double* fe_out, double* energy_out, double* grad_e,
                          int* flags, cudaStream_t st) {
   if (n_el == 0) return 0;
-  const int grid = grid_for(n_el, 1, 128, 16);
-  element_force_kernel<<<grid, 128, 0, st>>>(n_el, nodes, conn, props, u, stride, fe_out, energy_out, grad_e, flags);
+  element_force_kernel<<<el_grid(n_el), kElWarps * 32, 0, st>>>(n_el, nodes, conn, props, u, stride, fe_out, energy_out, grad_e, flags);
   WN_CUDA(cudaGetLastError());
   return 0;
 }
@@ -827,8 +983,7 @@ int launch_stress(int64_t n_el, int64_t n_nodes, const double* nodes, const int3
                   const double* u, const int64_t* inc_ptr, const int32_t* inc_ea, double* cell_sig, double* cell_vm,
                   double* nodal_vm, cudaStream_t st) {
   if (n_el > 0) {
-    const int grid = grid_for(n_el, 1, 128, 16);
-    stress_kernel<<<grid, 128, 0, st>>>(n_el, nodes, conn, props, u, cell_sig, cell_vm, nullptr, nullptr);
+    stress_kernel<<<el_grid(n_el), kElWarps * 32, 0, st>>>(n_el, nodes, conn, props, u, cell_sig, cell_vm, nullptr, nullptr);
     WN_CUDA(cudaGetLastError());
   }
   if (n_nodes > 0) {
@@ -842,8 +997,7 @@ int launch_stress(int64_t n_el, int64_t n_nodes, const double* nodes, const int3
 int launch_gp_stress(int64_t n_el, const double* nodes, const int32_t* conn, const double* props, const double* u,
                      double* gp_sig, double* gp_vm, cudaStream_t st) {
   if (n_el == 0) return 0;
-  const int grid = grid_for(n_el, 1, 128, 16);
-  stress_kernel<<<grid, 128, 0, st>>>(n_el, nodes, conn, props, u, nullptr, nullptr, gp_sig, gp_vm);
+  stress_kernel<<<el_grid(n_el), kElWarps * 32, 0, st>>>(n_el, nodes, conn, props, u, nullptr, nullptr, gp_sig, gp_vm);
   WN_CUDA(cudaGetLastError());
   return 0;
 }
