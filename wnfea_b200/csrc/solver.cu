@@ -1162,14 +1162,14 @@ __global__ void __launch_bounds__(kThreads) k_team_rows(int64_t n_rows, const in
 // warp-per-row kernels.  Measured (FP32, event-timed, warp-per-row or streamed -> teams):
 //   no pack: 413 blocks, 130 MB  43 -> 33 us; 343, 20 MB  21 -> 12 us; restrictions of 27 / 2.5 MB
 //            45 -> 14 and 26 -> 10 us;
-//   packed:  243, 76 MB  38 -> 24 us; 100, 30 MB  16 -> 15 us; but 134, 300 MB  76 -> 78 us and 105
-//            (6x3), 140 MB  33 -> 42 us: a pack of more than L2's share streams better until a row
+//   packed:  243, 76 MB  38 -> 24 us; but 134, 300 MB  76 -> 78 us, 105 (6x3), 140 MB  33 -> 42 us, and
+//            100, 30 MB  10.4 -> 11.8 us on the I-beam's level 2 (its solve 31.9 -> 33.1 ms: the streamed
+//            kernels before and after it lose their overlap too): a pack streams better until a row
 //            fills most of a tile.
-static int team_width(int64_t n_rows, int64_t nnzb, int block_bytes, bool packed) {
+static int team_width(int64_t n_rows, int64_t nnzb, bool packed) {
   if (n_rows <= 0) return 0;
   const double avg = (double)nnzb / (double)n_rows;
-  const bool big = (double)nnzb * block_bytes > 48e6;
-  if (avg < (packed ? (big ? 192.0 : 96.0) : 64.0)) return 0;
+  if (avg < (packed ? 192.0 : 64.0)) return 0;
   return avg >= 160.0 ? 8 : 4;
 }
 
@@ -1177,7 +1177,7 @@ template <int BC, typename T, typename XF, typename EPI>
 static bool launch_team_rows(int64_t n_rows, int64_t nnzb, bool packed, const int32_t* rp, const int32_t* ci,
                              const T* av, XF xf, EPI epi, double* part, const PcgScalars* S, cudaStream_t st,
                              int* grid_out) {
-  const int w = team_width(n_rows, nnzb, 6 * BC * (int)sizeof(T), packed);
+  const int w = team_width(n_rows, nnzb, packed);
   if (w == 0) return false;
   auto go = [&](auto kern, int rows_per_cta) {
     const int g = resident_grid(kern, kThreads, (n_rows + rows_per_cta - 1) / rows_per_cta);
