@@ -453,58 +453,137 @@ __global__ void __launch_bounds__(kSymThreads) ks_gemm_pattern(DMat A, const int
   }
 }
 
-// C(i, J) = sum over A(i,:) in order of A(i,k) B(k, J); nzflag = the block is not all zero.  A warp per
-// block of C: a lane per block of A's row searches B's sorted row for J, 32 searches at a time;
-// the blocks found are multiplied in order, a lane per entry of C's block.  (A thread per block runs
-// the searches one after the other and reads every block of A and B by itself: 2.0 ms per
-// 6x6 product on the levels of a 42,000-node matrix against 1.6.)
-template <int AR, int AK, int BC>
-__global__ void __launch_bounds__(kT) ks_gemm_values(DMat A, const int32_t* __restrict__ brp,
-                                                     const int32_t* __restrict__ bci, const double* __restrict__ bv,
-                                                     const int32_t* __restrict__ crow,
-                                                     const int32_t* __restrict__ cci, int64_t nnz,
-                                                     double* __restrict__ cv, uint8_t* __restrict__ nzflag) {
-  constexpr int NE = AR * BC, EL = (NE + 31) / 32;
-  const int lane = threadIdx.x & 31;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  int r[EL], t[EL];
+// C(i, J) = sum over A(i,:) in order of A(i,k) B(k, J); nzflag = the block is not all zero.  A CTA per
+// row of C, 32 blocks of A's row at a time: A's values go to shared memory, and every block of B's
+// rows j = A.ci[k] finds its column among C's (a search in shared memory that always hits) and notes
+// its place in a table by (column of C, k).  Then 8 lanes (4 for 3-row blocks) take a block of C each
+// and run through its k in order, three rows by two columns per lane, so that a block of B is read by
+// 16-byte loads, once per product; the sums wait in C between the runs of k.  The columns of C go
+// in runs of `cols` <= kCols, shared out over grid y.
+// Bound by the loads of B's blocks (33 M products of 6x6 blocks on level 1 of a 42,000-node matrix, 9.6 GB
+// through L1).  A warp per block of C that searched B's row for J under every k did three searches
+// in global memory per product: the six products of that matrix took 9.2 ms against 5.2.
+template <int AR, int AK, int BC, int kThreads, int kCols>
+__global__ void __launch_bounds__(kThreads) ks_gemm_values(DMat A, const int32_t* __restrict__ brp,
+                                                           const int32_t* __restrict__ bci,
+                                                           const double* __restrict__ bv,
+                                                           const int32_t* __restrict__ crp,
+                                                           const int32_t* __restrict__ cci, int cols,
+                                                           double* __restrict__ cv, uint8_t* __restrict__ nzflag) {
+  constexpr int NE = AR * BC, NA = AR * AK, NAP = NA | 1, TPR = BC / 2, LANES = AR / 3 * TPR, GL = LANES <= 4 ? 4 : 8;
+  static_assert(AR % 3 == 0 && BC % 2 == 0 && LANES <= GL, "three rows by two columns per lane");
+  __shared__ __align__(16) uint16_t place[kCols][32];  // B block (offset in its row) of (column, k), 0xffff: none
+  __shared__ double sa[32 * NAP];
+  __shared__ int32_t scol[kCols], sb[32], off[33];
+  const int tid = threadIdx.x, lane = tid & 31, gl = tid % GL, grp = tid / GL;
+  const unsigned gmask = ((1u << GL) - 1u) << (lane & ~(GL - 1));
+  const int r0 = min(gl / TPR, AR / 3 - 1) * 3, t0 = gl % TPR * 2;
+  const bool mine = gl < LANES;
+  for (int64_t i = blockIdx.x; i < A.n_rows; i += gridDim.x) {
+    const int32_t c_end = crp[i + 1], a_beg = A.rp[i], a_end = A.rp[i + 1];
+    for (int32_t c0 = crp[i] + blockIdx.y * cols; c0 < c_end; c0 += gridDim.y * cols) {
+      const int nc = min(cols, c_end - c0);
+      for (int c = tid; c < nc; c += kThreads) scol[c] = cci[c0 + c];
+      for (int32_t base = a_beg; base == a_beg || base < a_end; base += 32) {
+        const int nk = min(32, a_end - base);
+        for (int w = tid; w < nc * 4; w += kThreads)
+          reinterpret_cast<uint4*>(place)[w] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        if (tid < 32) {  // off[k]: blocks of B's rows before the k-th
+          int len = 0;
+          if (tid < nk) {
+            const int32_t j = A.ci[base + tid];
+            sb[tid] = brp[j];
+            len = brp[j + 1] - sb[tid];
+          }
+          int sum = len;
 #pragma unroll
-  for (int u = 0; u < EL; ++u) {
-    const int e = min(lane + 32 * u, NE - 1);
-    r[u] = e / BC;
-    t[u] = e % BC;
-  }
-  for (int64_t q = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; q < nnz; q += nw) {
-    const int64_t i = crow[q];
-    const int32_t J = cci[q], k1 = A.rp[i + 1];
-    double acc[EL] = {};
-    for (int32_t base = A.rp[i]; base < k1; base += 32) {
-      int32_t p_mine = -1;
-      if (base + lane < k1) {
-        const int32_t j = A.ci[base + lane];
-        p_mine = find_col(bci, brp[j], brp[j + 1], J);
-      }
-      unsigned hit = __ballot_sync(0xffffffffu, p_mine >= 0);
-      while (hit) {
-        const int l = __ffs(hit) - 1;
-        hit &= hit - 1;
-        const int64_t k = base + l;
-        const double* b = bv + (int64_t)__shfl_sync(0xffffffffu, p_mine, l) * AK * BC;
+          for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+          }
+          off[tid + 1] = sum;
+          if (tid == 0) off[0] = 0;
+        }
+        for (int w = tid; w < nk * NA; w += kThreads) {
+          int k, m;  // along the values as they are stored
+          if (A.stride) {
+            m = w / nk;
+            k = w - m * nk;
+          } else {
+            k = w / NA;
+            m = w - k * NA;
+          }
+          sa[k * NAP + m] = A.at(base + k, m / AK, m % AK);
+        }
+        __syncthreads();
+        const int n_cand = off[32];
+#pragma unroll 2
+        for (int w = tid; w < n_cand; w += kThreads) {
+          int k = 0;
 #pragma unroll
-        for (int u = 0; u < EL; ++u)
+          for (int o = 16; o > 0; o >>= 1)
+            if (off[k + o] <= w) k += o;
+          const int q = w - off[k];
+          const int32_t c = bci[sb[k] + q];
+          int lo = 0, hi = nc;
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (scol[mid] < c)
+              lo = mid + 1;
+            else
+              hi = mid;
+          }
+          if (lo < nc && scol[lo] == c) place[lo][k] = (uint16_t)q;
+        }
+        __syncthreads();
+        for (int c = grp; c < nc; c += kThreads / GL) {
+          unsigned hit = 0;  // the k of this block, from the lane's 32 / GL table entries
 #pragma unroll
-          for (int m = 0; m < AK; ++m) acc[u] = fma(A.at(k, r[u], m), b[m * BC + t[u]], acc[u]);
+          for (int e = 0; e < 16 / GL; ++e) {
+            const uint32_t two = reinterpret_cast<const uint32_t*>(place[c])[gl * (16 / GL) + e];
+            hit |= ((two & 0xffffu) != 0xffffu ? 1u : 0u) << (2 * e) | ((two >> 16) != 0xffffu ? 2u : 0u) << (2 * e);
+          }
+          hit = __reduce_or_sync(gmask, hit << (gl * (32 / GL)));
+          double* out = cv + (int64_t)(c0 + c) * NE + r0 * BC + t0;
+          double acc[3][2] = {};
+          if (base > a_beg && mine)
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+              const double2 v = *reinterpret_cast<const double2*>(out + r * BC);
+              acc[r][0] = v.x;
+              acc[r][1] = v.y;
+            }
+          while (hit) {
+            const int k = __ffs(hit) - 1;
+            hit &= hit - 1;
+            const double* bk = bv + ((int64_t)sb[k] + place[c][k]) * (AK * BC) + t0;
+            const double* ak = sa + k * NAP + r0 * AK;
+            double2 bm[AK];
+#pragma unroll
+            for (int m = 0; m < AK; ++m) bm[m] = *reinterpret_cast<const double2*>(bk + m * BC);
+#pragma unroll
+            for (int m = 0; m < AK; ++m)
+#pragma unroll
+              for (int r = 0; r < 3; ++r) {
+                acc[r][0] = fma(ak[r * AK + m], bm[m].x, acc[r][0]);
+                acc[r][1] = fma(ak[r * AK + m], bm[m].y, acc[r][1]);
+              }
+          }
+          bool nz = false;
+          if (mine)
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+              *reinterpret_cast<double2*>(out + r * BC) = make_double2(acc[r][0], acc[r][1]);
+              nz = nz || acc[r][0] != 0.0 || acc[r][1] != 0.0;
+            }
+          if (base + 32 >= a_end) {
+            const unsigned any = __ballot_sync(gmask, nz) & gmask;
+            if (gl == 0) nzflag[c0 + c] = any ? 1 : 0;
+          }
+        }
+        __syncthreads();
       }
     }
-    bool nz = false;
-#pragma unroll
-    for (int u = 0; u < EL; ++u)
-      if (lane + 32 * u < NE) {
-        cv[q * NE + lane + 32 * u] = acc[u];
-        nz = nz || acc[u] != 0.0;
-      }
-    const bool any = __any_sync(0xffffffffu, nz);
-    if (lane == 0) nzflag[q] = any ? 1 : 0;
   }
 }
 
@@ -802,7 +881,7 @@ int aggregate_device(const DMat& A, const DArray<double>& nrm, double theta, con
 template <int AR, int AK, int BC>
 int gemm(const DMat& A, const DevBsr& B, DevBsr& C, std::vector<int32_t>& h_rp) {
   const int64_t n = A.n_rows;
-  DArray<int32_t> cnt, rp_t, ci_t, row_t;
+  DArray<int32_t> cnt, rp_t, ci_t;
   DArray<int> err;
   WN_CHECK(cnt.alloc(std::max<int64_t>(n, 1)));
   WN_CHECK(err.alloc(1));
@@ -817,14 +896,17 @@ int gemm(const DMat& A, const DevBsr& B, DevBsr& C, std::vector<int32_t>& h_rp) 
   std::vector<int32_t> h_rp_t;
   WN_CHECK(scan_counts(cnt, n, rp_t, h_rp_t, &nnz));
   WN_CHECK(ci_t.alloc(std::max<int64_t>(nnz, 1)));
-  WN_CHECK(row_t.alloc(std::max<int64_t>(nnz, 1)));
   ks_gemm_pattern<<<gs, kSymThreads>>>(A, B.rp.p, B.ci.p, nullptr, rp_t.p, ci_t.p, err.p);
-  ks_block_rows<<<grid_for(n, 32, kT, 16), kT>>>(n, rp_t.p, row_t.p);
   DArray<double> v_t;
   DArray<uint8_t> flags;
   WN_CHECK(v_t.alloc(std::max<int64_t>(nnz, 1) * AR * BC));
   WN_CHECK(flags.alloc(std::max<int64_t>(nnz, 1)));
-  ks_gemm_values<AR, AK, BC><<<grid_for(nnz, 32, kT, 16), kT>>>(A, B.rp.p, B.ci.p, B.v64.p, row_t.p, ci_t.p, nnz, v_t.p, flags.p);
+  // rows of the fine product have a few dozen columns: small CTAs; the few rows of a coarse product
+  // (hundreds of columns) are cut into runs of 64 columns to fill the SMs
+  constexpr int kThreads = AR == 3 ? 64 : 256, kCols = AR == 3 ? 64 : 256;
+  const bool few = n < (int64_t)kNumSMs * 8;
+  ks_gemm_values<AR, AK, BC, kThreads, kCols><<<dim3(gs, few ? 4 : 1), kThreads>>>(
+      A, B.rp.p, B.ci.p, B.v64.p, rp_t.p, ci_t.p, few ? 64 : kCols, v_t.p, flags.p);
   WN_CUDA(cudaGetLastError());
   return compact_into(n, AR, BC, B.n_cols, nnz, rp_t, ci_t, v_t, flags, C, h_rp);
 }
