@@ -76,6 +76,51 @@ struct XD0 {  // d0_j = dinv_j b_j / theta   (first Chebyshev step from a zero g
   T inv_theta;
   __device__ __forceinline__ T operator()(int64_t j) const { return dinv[j] * b[j] * inv_theta; }
 };
+// The same functors for vectors of 6-DOF nodes, a node's six values in three 8-byte (FP32) or 16-byte
+// (FP64) loads: the gathers of 32 scattered nodes are most of a 6x6 level's L1 wavefronts, and a
+// wavefront serves a cache line whatever the width of the load.
+// The 162,000-element design step 29.0 -> 28.3 ms, the 97-slice FP64 solve 14.3 -> 14.1 ms, same bits.
+template <typename T>
+__device__ __forceinline__ void load6(const T* __restrict__ x, int64_t node, T (&v)[6]) {
+  using V2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+  const V2* p = reinterpret_cast<const V2*>(x + node * 6);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const V2 a = p[i];
+    v[2 * i] = a.x;
+    v[2 * i + 1] = a.y;
+  }
+}
+template <typename T>
+struct XLoad6 {
+  static constexpr bool kLoadsBlocks = true;
+  const T* __restrict__ x;
+  __device__ __forceinline__ void block(int64_t node, T (&v)[6]) const { load6(x, node, v); }
+};
+template <typename T>
+struct XD06 {
+  static constexpr bool kLoadsBlocks = true;
+  const T* __restrict__ b;
+  const T* __restrict__ dinv;
+  T inv_theta;
+  __device__ __forceinline__ void block(int64_t node, T (&v)[6]) const {
+    T d[6];
+    load6(b, node, v);
+    load6(dinv, node, d);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) v[c] = d[c] * v[c] * inv_theta;
+  }
+};
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+template <typename T>
+static bool loads6(const XLoad<T, T>& f) { return aligned16(f.x); }
+template <typename T>
+static bool loads6(const XD0<T>& f) { return aligned16(f.b) && aligned16(f.dinv); }
+template <typename T>
+static XLoad6<T> six(const XLoad<T, T>& f) { return {f.x}; }
+template <typename T>
+static XD06<T> six(const XD0<T>& f) { return {f.b, f.dinv, f.inv_theta}; }
+
 template <typename T>
 struct XD0U {  // the same with a unit diagonal (the FP16 V-cycle's equilibrated fine level)
   const T* __restrict__ b;
@@ -1133,8 +1178,7 @@ __global__ void __launch_bounds__(kThreads) k_team_rows(int64_t n_rows, const in
     for (int r = 0; r < BR; ++r) acc[r] = T(0);
     while (b < e) {
       T x[BC];
-#pragma unroll
-      for (int c = 0; c < BC; ++c) x[c] = xf((int64_t)col * BC + c);
+      load_block<BC>(xf, col, x);
 #pragma unroll
       for (int r = 0; r < BR; ++r)
 #pragma unroll
@@ -1195,22 +1239,27 @@ static bool launch_team_rows(int64_t n_rows, int64_t nnzb, bool packed, const in
 template <int BR, int BC, typename T, bool SC = false>
 static void level_spmv(const DevBsr& M, const StreamMat& Ms, const T* vals, const T* x, T* y, int accumulate,
                        PcgScalars* S, cudaStream_t st, const T* ys = nullptr) {
-  if constexpr (BR == 6 && !SC) {
-    if (launch_team_rows<BC, T>(M.n_rows, M.nnzb, Ms.packed, M.rp.p, M.ci.p, vals, XLoad<T, T>{x},
-                                EpiLevel<T, false>{y, accumulate, nullptr}, nullptr, S, st, nullptr))
-      return;
-  }
-  if constexpr (BR == 6 && BC == 6) {  // short rows (the prolongations): 8 lanes per row
-    if (M.nnzb < 16 * M.n_rows) {
-      if (launch_stream_rows<T, 6, 6, XLoad<T, T>, EpiLevel<T, SC>, StreamShort66<T>>(
-              Ms, XLoad<T, T>{x}, EpiLevel<T, SC>{y, accumulate, ys}, nullptr, S, st, nullptr))
-        return;
-      level_spmv_rows<BR, BC, T>(M, vals, x, y, accumulate, S, st, SC ? ys : nullptr);
-      return;
+  // x: a level's vector of the workspace (an allocation's start), or the general kernel below
+  auto streamed = [&](auto xf) {
+    if constexpr (BR == 6 && !SC) {
+      if (launch_team_rows<BC, T>(M.n_rows, M.nnzb, Ms.packed, M.rp.p, M.ci.p, vals, xf,
+                                  EpiLevel<T, false>{y, accumulate, nullptr}, nullptr, S, st, nullptr))
+        return true;
     }
+    const EpiLevel<T, SC> epi{y, accumulate, ys};
+    if constexpr (BR == 6 && BC == 6) {  // short rows (the prolongations): 8 lanes per row
+      if (M.nnzb < 16 * M.n_rows)
+        return launch_stream_rows<T, 6, 6, decltype(xf), EpiLevel<T, SC>, StreamShort66<T>>(Ms, xf, epi, nullptr, S,
+                                                                                           st, nullptr);
+    }
+    return launch_stream_rows<T, BR, BC>(Ms, xf, epi, nullptr, S, st, nullptr);
+  };
+  const XLoad<T, T> xl{x};
+  if constexpr (BC == 6) {
+    if (loads6(xl) && streamed(six(xl))) return;
+  } else {
+    if (streamed(xl)) return;
   }
-  if (launch_stream_rows<T, BR, BC>(Ms, XLoad<T, T>{x}, EpiLevel<T, SC>{y, accumulate, ys}, nullptr, S, st, nullptr))
-    return;
   level_spmv_rows<BR, BC, T>(M, vals, x, y, accumulate, S, st, SC ? ys : nullptr);
 }
 
@@ -1362,10 +1411,14 @@ static int vcycle(Solid* s, AmgHierarchy& H, SolverWork& W, int lvl, const T* b,
         return true;
       } else {
         if constexpr (BS == 6) {
-          if (launch_team_rows<BS, T>(nr, lvl == 0 ? s->nnzb : L.A.nnzb, stream, rp, ci, av, xf, epi, prt, S, st, gout))
+          if (!loads6(xf)) return false;  // the register row kernels load value by value
+          const auto x6 = six(xf);
+          if (launch_team_rows<BS, T>(nr, lvl == 0 ? s->nnzb : L.A.nnzb, stream, rp, ci, av, x6, epi, prt, S, st, gout))
             return true;
+          return stream && launch_stream_rows<T, BS, BS>(Am, x6, epi, prt, S, st, gout);
+        } else {
+          return stream && launch_stream_rows<T, BS, BS>(Am, xf, epi, prt, S, st, gout);
         }
-        return stream && launch_stream_rows<T, BS, BS>(Am, xf, epi, prt, S, st, gout);
       }
     };
     const T c1 = deg >= 2 ? (T)L.c1[0] : T(0), c2 = deg >= 2 ? (T)L.c2[0] : T(0);

@@ -552,6 +552,23 @@ __device__ __forceinline__ T value_as(TV v) {
     return (T)v;
 }
 
+// whether an x functor loads a block column's DOFs at once: block(col, out)
+template <typename XF, typename = void>
+struct LoadsBlocks : std::false_type {};
+template <typename XF>
+struct LoadsBlocks<XF, std::void_t<decltype(XF::kLoadsBlocks)>> : std::true_type {};
+
+// x_j = xf(j) of block column col
+template <int BC, typename T, typename XF>
+__device__ __forceinline__ void load_block(const XF& xf, int64_t col, T (&x)[BC]) {
+  if constexpr (LoadsBlocks<XF>::value) {
+    xf.block(col, x);
+  } else {
+#pragma unroll
+    for (int c = 0; c < BC; ++c) x[c] = xf(col * BC + c);
+  }
+}
+
 // The row engine: y-rows of A x with G lanes per block row (lane l taking the row's blocks
 // l, l + G, ...; U blocks in flight per lane, R rows per lane group), for every row DOF
 // i = BR row + c of the CTA's tiles the owning lane (c < BR <= G) calls pre = epi.load(i) before
@@ -615,9 +632,7 @@ __device__ __forceinline__ double stream_rows_v(const PackTile* __restrict__ til
 #pragma unroll
         for (int q = 0; q < R; ++q)
 #pragma unroll
-          for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int c = 0; c < BC; ++c) xv[q][u][c] = xf((int64_t)col[q][u] * BC + c);
+          for (int u = 0; u < U; ++u) load_block<BC>(xf, col[q][u], xv[q][u]);
 #pragma unroll
         for (int q = 0; q < R; ++q)
 #pragma unroll
