@@ -126,7 +126,7 @@ int wn_solid_set_stream(void* h, int enable);
 /* Batched solves (wn_solve_multi*): the FP32 fine-level passes with each row tile's x slice
  * (the 32 cases of the tile's column nodes) staged in shared memory (enable != 0), or the
  * register row kernels gathering x through L1/L2 (0, the default: on the 1M-DOF I-beam the
- * staged passes are slower, 312 vs 270 ms per 32-case batch).  The same arithmetic in the same
+ * staged passes are slower: 312 ms per 32-case batch).  The same arithmetic in the same
  * order: the row products are bitwise the same.  Synchronises. */
 int wn_solid_set_batch_staging(void* h, int enable);
 /* Status word of the streamed fine-matrix products of wn_spmv_solid_device: WN_OK, or
@@ -245,7 +245,8 @@ typedef struct wn_solve_params {
   int chunk;          /* iterations per CUDA-graph replay / host convergence check    */
   int use_graph;      /* 1 = replay captured chunks as a CUDA graph                   */
   int profile;        /* 1 = time every kernel of this solve with CUDA events (graphs
-                         off; read back with wn_solve_profile); 0 = normal          */
+                         off; read back with wn_solve_profile; small systems run
+                         the same kernels one by one); 0 = normal */
 } wn_solve_params;
 
 typedef struct wn_solve_stats {
@@ -294,8 +295,8 @@ int wn_beam_linear_system(void* beam, void** out_handle);
 
 /* Multi-right-hand-side solve (no reference counterpart: the reference solves load cases one
  * solve_c3d10_pcg call at a time, solid_solver.py:197-308).  F, U: row-major n x n_rhs
- * (n = 3 n_nodes, load case j in column j).  Cases are solved in batches of 32 sharing every
- * matrix read; each case keeps its own PCG recurrence and stops at its own
+ * (n = 3 n_nodes, load case j in column j).  Cases are solved in batches of 8, 16 or 32 (the
+ * narrowest that holds them) sharing every matrix read; each case keeps its own PCG recurrence and stops at its own
  * ||F_j - K U_j|| <= rtol ||F_j|| (FP64 true residual).  precision 0: FP64 V-cycle; 1: FP32
  * V-cycle inside the FP64 PCG.  stats: iterations = batched iterations summed over batches,
  * status = worst case, rel_res = largest case residual.  case_iters / case_rel_res: optional

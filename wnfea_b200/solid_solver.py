@@ -127,7 +127,7 @@ def solve_c3d10_multi(
     """Several load cases at once -> (U, stats); F is (n, k), one load case per column.
 
     No reference counterpart: the reference runs solve_c3d10_pcg once per load case
-    (solid_solver.py:197-308).  Here the cases go through the GPU in batches of 32 that share
+    (solid_solver.py:197-308).  Here the cases go through the GPU in batches of up to 32 that share
     every matrix read, each case with its own PCG recurrence and its own stopping test on the
     FP64 true residual.  ``precision``: "fp64" or "mixed_fp32" (FP32 V-cycle in FP64 PCG).
     stats adds ``case_iterations`` and ``case_rel_res`` (arrays of k).

@@ -136,8 +136,8 @@ class SolidSystem:
 
     def solve_multi(self, F: np.ndarray, rtol: float = 1e-8, max_iter: int = 2000, precond: int = 2,
                     precision: int = 1, max_outer: int = 10, chunk: int = 8, use_graph: bool = True):
-        """Solve K U = F for the load cases in the columns of F (n x k, host) in batches of 32
-        sharing every matrix read; returns (U, stats dict with per-case 'case_iterations' and
+        """Solve K U = F for the load cases in the columns of F (n x k, host) in batches of up
+        to 32 sharing every matrix read; returns (U, stats dict with per-case 'case_iterations' and
         'case_rel_res')."""
         F = np.ascontiguousarray(F, dtype=np.float64)
         if F.ndim == 1:
