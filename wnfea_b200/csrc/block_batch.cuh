@@ -788,6 +788,7 @@ __device__ __forceinline__ void batch_stream_rows(const BView& m, const XF& xf, 
 #pragma unroll
       for (int r = 0; r < 3; ++r) epi.store(i0 + r, l, pre[r], acc[r], dot);
     }
+    return true;
   };
   stream_pipeline<T, 9, Cfg>(m.tiles, m.n_tiles, m.pack, smem, &S->status, &S->done, m.ctl, skipped, hook, body);
 }
