@@ -4,15 +4,16 @@
 // its time in the block products of the Galerkin operator (A P, then R (A P)), in the power
 // iterations for rho(D^-1 A) and in the smoothed prolongator (I - w D^-1 A) P_tent -- all of
 // them passes over matrices that already live in HBM.  Here each level runs:
-//   device: 1/diag(A), rho(D^-1 A) by power iteration, the Frobenius norm of every block;
-//   host:   the greedy aggregation from those norms and the per-aggregate QR of the near-null
-//           space (sequential, and cheap: a few percent of the host builder's time);
+//   device: 1/diag(A), rho(D^-1 A) by power iteration, the Frobenius norm of every block and from it
+//           which blocks are strong; pass 2 of the greedy aggregation (joining);
+//   host:   passes 1 and 3 of the aggregation and the per-aggregate QR of the near-null space
+//           (sequential, and cheap: a few percent of the host builder's time);
 //   device: P = (I - w D^-1 A) P_tent, R = P^T, A P, A_c = R (A P), symmetrised.
 // Every device product is deterministic and follows the host builder's summation order (per
 // output block: the left factor's row in order, then the block product r, s, t), and blocks that
 // come out all zero are dropped as the host builder drops them.  Each sparse product is a
 // symbolic pass (the sorted unique output columns of each row, found with a hash set in shared
-// memory), a numeric pass (one thread per output block) and a compaction pass.
+// memory), a numeric pass (one CTA per output row) and a compaction pass.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
