@@ -1,0 +1,55 @@
+"""Small systems without AMG: the one-kernel solve adds its dot products in the order of the launched kernels
+(which a profiled solve runs), so that iterates, counts and residuals are theirs bit for bit, also where
+the solve stops at its iteration limit, and no solve runs twice."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from wnfea_b200.mesh import generate_c3d10_kuhn_block, tip_load_cases
+from wnfea_b200.model import solid_fixed_dofs
+from wnfea_b200.solid_solver import assemble_c3d10_sparse_3dof
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(nx, ny, nz, seed):
+    m, _ = generate_c3d10_kuhn_block(0.05 * nx, 0.05 * ny, 0.05 * nz, nx, ny, nz)
+    K, _, _ = assemble_c3d10_sparse_3dof(m)
+    F = tip_load_cases(m.mesh_nodes, 1, seed=seed)[:, 0]
+    F[np.asarray(solid_fixed_dofs(m), dtype=np.int64)] = 0.0
+    return K.system, np.ascontiguousarray(F)
+
+
+def _same(s, F, **kw):
+    u, st = s.solve(F, **kw)
+    v, sv = s.solve(F, profile=True, **kw)
+    assert np.array_equal(u, v)
+    assert st["iterations"] == sv["iterations"] and st["status"] == sv["status"]
+    assert st["rel_res"] == sv["rel_res"]
+    return st
+
+
+# 27 nodes (CTAs without rows), 99, 585, 603 (slender: two outer passes), 1,025 and 1,105 (the matrix in shared
+# memory), 1,815 and 2,023 (in L2)
+@pytest.mark.parametrize("cells", [(1, 1, 1), (5, 1, 1), (6, 4, 2), (25, 1, 1), (20, 2, 2), (8, 6, 2), (7, 5, 5),
+                                   (8, 8, 3)])
+@pytest.mark.parametrize("precond", [0, 1, 3])
+def test_same_bits_as_the_launched_kernels(cells, precond):
+    s, F = _system(*cells, seed=sum(cells))
+    st = _same(s, F, rtol=1e-6, max_iter=2000, precond=precond)
+    if precond:
+        assert st["status"] == 0
+
+
+# bars that the default 2,000 iterations do not bring to 1e-6, and a limit of a few iterations
+@pytest.mark.parametrize("cells,limit", [((37, 1, 1), 2000), ((34, 2, 1), 2000), ((20, 2, 2), 3)])
+@pytest.mark.parametrize("precond", [0, 1])
+def test_iteration_limit_returns_the_iterate_once(cells, limit, precond):
+    s, F = _system(*cells, seed=7)
+    st = _same(s, F, rtol=1e-6, max_iter=limit, precond=precond)
+    assert st["status"] == -5 and st["iterations"] == limit
+    assert st["kernel_launches"] < 20
+    st = s.solve(F, rtol=1e-6, max_iter=limit, precond=precond, precision=1)[1]
+    assert st["status"] == -5 and st["iterations"] == limit and st["kernel_launches"] < 20

@@ -141,6 +141,9 @@ struct SolverWork {
   DArray<float> binv32;
   PcgVecs<double> p64;
   PcgVecs<float> p32;
+  // small systems (small_solve.cu): the plan of the pattern, made by the first solve (small_tiles > 0)
+  DArray<int4> small_plan;
+  int small_tiles = 0, small_rows = 0, small_blocks = 0, small_units = 0;
   // the FP16 V-cycle (solve precision 3): set for the solve's duration; s = diag(K)^-1/2 of the
   // current matrix (FP64 for the FP16 pack, FP32 for the vectors) and q = 1 / s
   bool half = false;

@@ -2,22 +2,27 @@
 //
 // A system of a few thousand nodes gives each of an iteration's kernels (five with point Jacobi, nine
 // with a two-level V-cycle) a microsecond of work and three to five of launch, ramp-up and
-// dependence: 15.8 us per point-Jacobi and 35 us per AMG iteration at 1,025 nodes, whatever the matrix.
+// dependence, whatever the matrix (small_system has the figures).
 // Here the stages of an iteration are the phases of one persistent kernel, separated by the
 // hardware barrier of a thread-block cluster (16 CTAs on 16 SMs of one GPC: co-scheduled by the
 // launch, no spinning).  What bounds it is the chain of phases, so nothing on it goes through L2
 // that need not:
 //   * every CTA holds a copy of the gathered vectors in its shared memory; a CTA computes its run of
 //     rows and stores the result into all 16 copies before the barrier.  (Gathering through L2
-//     instead, two round trips per phase, took 11 and 35 us per iteration.)
+//     instead, two round trips per phase, took 11 and 35 us per iteration at 1,025 nodes.)
 //   * p = z + beta p is formed by every CTA for itself, so only z travels;
-//   * x, r and q of the CTA's own rows stay in its shared memory, as do their matrix blocks when they
-//     fit (about 2,000 FP64 blocks per CTA); otherwise the blocks are read from L2, which does not
-//     depend on any phase;
+//   * x, r and q of the CTA's own DOFs stay in its registers or shared memory, as do its matrix
+//     blocks when they fit; otherwise the blocks are read from L2, which does not depend on any
+//     phase;
 //   * dot products: one partial per warp, stored into every CTA before the barrier; each warp adds
-//     the 256 partials in the same order, so all threads take the same alpha, beta and decisions.
+//     the partials in the same order, so all threads take the same alpha, beta and decisions.
+// Two kernels: k_small_diag for no, point-Jacobi or block-Jacobi preconditioning, and k_small_amg
+// for a hierarchy of at most one level above its dense one.
 // The arithmetic is that of the launched kernels (solver.cu): FP64 Krylov vectors, matrix and dots;
-// the preconditioner in TM.  Sums run in another order.
+// the preconditioner in TM.  k_small_diag also adds its dot products in the launched kernels'
+// order: an unpreconditioned or Jacobi solve that stops at its iteration limit hundreds of
+// iterations from convergence (a slender bar) has an iterate that depends on that order in its third
+// digit, and a call's result must not depend on which kernels ran it.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -28,6 +33,7 @@
 #include "small_solve.h"
 #include "solid.h"
 #include "spmv.cuh"
+#include "stream.cuh"
 #include "wnfea_cuda.h"
 
 namespace cg = cooperative_groups;
@@ -40,23 +46,352 @@ constexpr int kLanes = 8;                   // lanes per block row
 constexpr int kGroups = kThreads / kLanes;  // rows of a CTA side by side
 constexpr int kTeam = 4, kTeams = kWarps / kTeam;  // warps per row of the restriction
 constexpr int64_t kMaxNodes = 2048;         // (small_system)
-constexpr size_t kSmemLimit = 214 * 1024;   // dynamic shared memory (11 KB are static)
+constexpr size_t kSmemLimit = 214 * 1024;   // dynamic shared memory (5 KB are static)
 
+__host__ __device__ constexpr size_t pad16(size_t bytes) { return (bytes + 15) & ~size_t(15); }
+
+// the run [i0, i1) of a vector, complete in this CTA's copy, into the other CTAs' copies (visible
+// after the next cluster barrier); i0 sizeof(T) is a multiple of 16
+template <int THREADS, typename T>
+__device__ __forceinline__ void publish_run(const cg::cluster_group& c, int rank, T* v, int64_t i0, int64_t i1) {
+  __syncthreads();  // the run is complete
+  const int64_t u0 = i0 * sizeof(T) / 16, u1 = (i1 * sizeof(T) + 15) / 16;
+  const int n = (int)(u1 - u0);
+  uint4* own = reinterpret_cast<uint4*>(v) + u0;
+  for (int k = threadIdx.x; k < n * (kCtas - 1); k += THREADS) {
+    const int peer = k / n, at = k - peer * n;
+    uint4* there = c.map_shared_rank(own, peer + (peer >= rank));
+    there[at] = own[at];
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// no, point-Jacobi or block-Jacobi preconditioning
+// ---------------------------------------------------------------------------------------
+// The dot products in the launched kernels' order:
+//   p . q   a tile of the streamed fine matrix is a CTA of eight consumer warps there, warp w taking the
+//           rows 4 w .. 4 w + 3 of every 32; such a warp's rows are a unit here, and the units are shared
+//           out evenly over the 16 CTAs.  A tile's eight sums are added as block_sum adds them,
+//           then the tiles' as reduce_parts does.
+//   r . r, r . z   a warp there takes 32 consecutive DOFs (block Jacobi, r . z: nodes) and a CTA eight
+//           such warps; so a CTA here owns whole runs of 32 nodes (96 DOFs) of x, r and z.
+// q = A p is stored by the warp that computes it into the shared memory of its owner.
+// Bound by the chain of phases: two cluster barriers with their sums, the row products and the copies of
+// z.  1,025 nodes 7.0 us per iteration (about as much as with sums in the cheapest order, 7.4 with an
+// earlier split of the rows); the part of the matrix that shared memory cannot hold is read from L2 by the
+// first units of a CTA, 2,025 nodes 12.7 us.
+constexpr int kDiagThreads = 512, kDiagWarps = kDiagThreads / 32;
+constexpr int kMaxTiles = 128;                  // (as many as one CTA of the update reduces in four warps)
+constexpr size_t kDiagSmemLimit = 226 * 1024;   // dynamic shared memory (no static)
+static_assert(kMaxNodes / kCtas * 3 <= kDiagThreads, "one owned DOF per thread");
+
+template <typename TM>
+struct DiagArgs {
+  int64_t n_nodes, nnzb;
+  const int32_t *rp, *ci;
+  const double* k64;
+  const TM* dinv;  // 1 / diag
+  const TM* binv;  // block Jacobi
+  int precond;
+  const double* b;
+  double* x;
+  const int4* plan;  // kCtas runs (first unit, end, first row, end), then the units (small_plan)
+  int slots;         // tiles rounded up to 32
+  int own_max, rows_max, units_max;
+  int slice_blocks;  // the last blocks of a CTA's run, in shared memory; those before are read from L2
+  double rtol;
+  int max_iter;
+  PcgScalars* S;
+};
+
+// first run of 32 nodes that CTA k owns
+__host__ __device__ __forceinline__ int64_t own_begin(int64_t n_nodes, int k) {
+  return (n_nodes + 31) / 32 * k / kCtas;
+}
+
+// dynamic shared memory of a CTA, in this order
+template <typename TM>
+struct DiagLayout {
+  size_t p, z, pq, rr, rz, q, units, kv, ci, rp, end;
+  __host__ __device__ DiagLayout(int64_t n_nodes, int slots, int own, int rows, int n_units, int slice) {
+    const size_t n = 3 * (size_t)n_nodes, bl = (size_t)slice;
+    p = 0;
+    z = p + pad16(n * 8);
+    pq = z + pad16(n * sizeof(TM));
+    rr = pq + 8 * (size_t)slots * 8;
+    rz = rr + 8 * 32 * 8;
+    q = rz + 8 * 32 * 8;
+    units = q + pad16(3 * (size_t)own * 8);
+    kv = units + 16 * (size_t)n_units;
+    ci = kv + pad16(9 * bl * 8);
+    rp = ci + pad16(bl * 4);
+    end = rp + pad16(4 * (size_t)(rows + 1));
+  }
+};
+
+// the sum of eight warps as block_sum adds them (its butterfly over lanes 0 .. 7), v[k * stride]
+__device__ __forceinline__ double sum8(const double* v, int stride) {
+  return ((v[0] + v[4 * stride]) + (v[2 * stride] + v[6 * stride])) +
+         ((v[stride] + v[5 * stride]) + (v[3 * stride] + v[7 * stride]));
+}
+
+// kWhole: every CTA's matrix blocks are in its shared memory
+template <typename TM, bool kWhole>
+__global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kDiagThreads, 1)
+    k_small_diag(const __grid_constant__ DiagArgs<TM> A) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const cg::cluster_group c = cg::this_cluster();
+  const int rank = (int)c.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t n = 3 * A.n_nodes, n_runs = (A.n_nodes + 31) / 32;
+  const DiagLayout<TM> lay(A.n_nodes, A.slots, A.own_max, A.rows_max, A.units_max,
+                           A.slice_blocks);
+  double* const p = reinterpret_cast<double*>(smem + lay.p);    // search direction, all DOFs
+  TM* const z = reinterpret_cast<TM*>(smem + lay.z);            // M^-1 r, all DOFs
+  double* const pq = reinterpret_cast<double*>(smem + lay.pq);  // [warp of a tile][tile]
+  double* const srr = reinterpret_cast<double*>(smem + lay.rr);  // [warp of a CTA][CTA] of the launched update
+  double* const srz = reinterpret_cast<double*>(smem + lay.rz);  // ... of the launched preconditioner
+  double* const q = reinterpret_cast<double*>(smem + lay.q);    // the owned DOFs of A p
+  // the owned DOFs, one per thread
+  const int64_t i0 = 96 * own_begin(A.n_nodes, rank), i1 = min(n, 96 * own_begin(A.n_nodes, rank + 1));
+  const int n_own = (int)(i1 - i0);
+  const bool own = tid < n_own;
+  const int64_t mine = i0 + tid;
+
+  // the matrix rows of the CTA's units
+  const int4 run = __ldg(A.plan + rank);
+  const int64_t c0 = run.z, c1 = run.w;
+  const int32_t q0 = __ldg(A.rp + c0);
+  const int cnt = __ldg(A.rp + c1) - q0;
+  int32_t* const rp = reinterpret_cast<int32_t*>(smem + lay.rp);
+  for (int64_t k = tid; k <= c1 - c0; k += kDiagThreads) rp[k] = __ldg(A.rp + c0 + k) - q0;
+  int4* const units = reinterpret_cast<int4*>(smem + lay.units);
+  for (int k = tid; k < run.y - run.x; k += kDiagThreads) units[k] = __ldg(A.plan + kCtas + run.x + k);
+  double* const sk = reinterpret_cast<double*>(smem + lay.kv);
+  int32_t* const sc = reinterpret_cast<int32_t*>(smem + lay.ci);
+  const int far = max(0, cnt - A.slice_blocks);  // blocks read from L2
+  for (int b = tid; b < cnt - far; b += kDiagThreads) {
+    sc[b] = __ldg(A.ci + q0 + far + b);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) sk[k * A.slice_blocks + b] = __ldg(A.k64 + k * A.nnzb + q0 + far + b);
+  }
+  const TM di = A.precond == 1 && own ? __ldg(A.dinv + mine) : TM(1);
+  for (int64_t i = tid; i < n; i += kDiagThreads) p[i] = 0.0;
+  for (int i = tid; i < 8 * A.slots; i += kDiagThreads) pq[i] = 0.0;  // units and warps without rows add zero
+  for (int i = tid; i < 8 * 32; i += kDiagThreads) srr[i] = srz[i] = 0.0;
+
+  // a warp's sum into place j of every CTA's partials
+  auto put = [&](double* part, int j, double v) {
+    const double s = warp_sum(v);
+    if (lane < kCtas) c.map_shared_rank(part, lane)[(j & 7) * 32 + (j >> 3)] = s;
+  };
+  // r . r (the thread's share in `rr`) and z = M^-1 r of the owned r with r . z; both sums
+  auto precondition = [&](double r, double rr, double& sum_rr, double& sum_rz) {
+    const int j0 = (int)(i0 / 32);  // the first launched warp of the owned DOFs
+    if (warp * 32 < n_own) put(srr, j0 + warp, rr);
+    if (A.precond == 3) {
+      if (own) q[tid] = r;  // (q is used up)
+      __syncthreads();
+      if (warp * 96 < n_own) {  // a node per thread
+        double dot = 0.0;
+        if (tid * 3 < n_own) {
+          TM rv[3];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) rv[j] = (TM)q[tid * 3 + j];
+          const TM* b = A.binv + (mine - tid) * 3 + (int64_t)tid * 9;
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            TM zk = TM(0);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) zk = fma(__ldg(b + k * 3 + j), rv[j], zk);
+            z[i0 + tid * 3 + k] = zk;
+            dot = fma((double)rv[k], (double)zk, dot);
+          }
+        }
+        put(srz, (int)(i0 / 96) + warp, dot);
+      }
+    } else {
+      const TM ri = (TM)r;
+      const TM zi = di * ri;
+      if (own) z[mine] = zi;
+      if (warp * 32 < n_own) put(srz, j0 + warp, (double)ri * (double)zi);
+    }
+    publish_run<kDiagThreads>(c, rank, z, i0, i1);
+    c.sync();
+    sum_rr = warp_sum(sum8(srr + lane, 32));
+    sum_rz = warp_sum(sum8(srz + lane, 32));
+  };
+  // q = A p of the CTA's units; p . q
+  auto product = [&]() {
+    const int grp = lane / kLanes, gl = lane % kLanes;
+    const int my_r = gl >> 1;  // (group_sum_transposed: row DOF r in the lanes 2 r, 2 r + 1)
+    const bool owner = (gl & 1) == 0 && my_r < 3;
+    // (to and fro over the warps: those with two units from L2 are not those with three)
+    for (int u0 = 0, turn = 0; u0 < run.y - run.x; u0 += kDiagWarps, turn ^= 1) {
+      const int u = u0 + (!kWhole && turn ? kDiagWarps - 1 - warp : warp);
+      if (u >= run.y - run.x) continue;
+      const int4 unit = units[u];  // first row, end of the tile, place of its sum
+      double dot = 0.0;
+      for (int base = unit.x; base < unit.y; base += 32) {
+        const int row = base + grp;
+        const bool active = row < unit.y;
+        double acc[3] = {0.0, 0.0, 0.0};
+        int b = 0, e = 0;
+        if (active) {
+          b = rp[row - c0] + gl;
+          e = rp[row - c0 + 1];
+        }
+        const int at = (16 * (row >> 5) + 15) / (int)n_runs;  // the CTA that owns the row's DOFs
+        // component k of block b at v[k * stride + b]; two blocks in flight, added in order
+        auto blocks = [&](const double* v, const int32_t* ci, int64_t stride) {
+          for (; b < e; b += 2 * kLanes) {
+            const bool two = b + kLanes < e;
+            const int b2 = two ? b + kLanes : b;
+            const double* xa = p + ci[b] * 3;
+            const double* xb = p + ci[b2] * 3;
+            double va[9], vb[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+              va[k] = v[k * stride + b];
+              vb[k] = v[k * stride + b2];
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+              for (int j = 0; j < 3; ++j) acc[r] = fma(va[r * 3 + j], xa[j], acc[r]);
+            if (two)
+#pragma unroll
+              for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) acc[r] = fma(vb[r * 3 + j], xb[j], acc[r]);
+          }
+        };
+        if (kWhole || __all_sync(0xffffffffu, !active || b - gl >= far))
+          blocks(sk - far, sc - far, A.slice_blocks);
+        else
+          blocks(A.k64 + q0, A.ci + q0, A.nnzb);
+        const double t = group_sum_transposed<3, kLanes>(acc, gl);
+        if (active && owner) {
+          const int64_t i = (int64_t)row * 3 + my_r;
+          c.map_shared_rank(q, at)[i - 96 * own_begin(A.n_nodes, at)] = t;
+          dot = fma(p[i], t, dot);
+        }
+      }
+      const double s = warp_sum(dot);
+      if (lane < kCtas) c.map_shared_rank(pq, lane)[unit.z] = s;
+    }
+    c.sync();
+    double w[kMaxTiles / 32];
+#pragma unroll
+    for (int g = 0; g < kMaxTiles / 32; ++g) w[g] = g * 32 < A.slots ? warp_sum(sum8(pq + g * 32 + lane, A.slots)) : 0.0;
+    return (w[0] + w[2]) + (w[1] + w[3]);
+  };
+
+  c.sync();  // every CTA of the cluster has started; its zeros are in place
+  double x = 0.0, r = own ? __ldg(A.b + mine) : 0.0, bb, rz;
+  precondition(r, r * r, bb, rz);
+  const double tol2 = A.rtol * A.rtol * bb;
+  double rr = bb, rz_prev = 0.0, alpha = 0.0;
+  int it = 0, status = 0;
+  bool done = false;
+  if (bb == 0.0 || !isfinite(bb)) {
+    done = true;
+    status = isfinite(bb) ? 0 : WN_EBREAKDOWN;
+  }
+  while (!done) {
+    const double beta = it == 0 ? 0.0 : rz / rz_prev;
+    for (int64_t i = tid; i < n; i += kDiagThreads) p[i] = fma(beta, p[i], (double)z[i]);
+    __syncthreads();
+    const double gamma = product();
+    alpha = rz / gamma;
+    if (!(gamma > 0.0) || !isfinite(alpha)) {
+      status = WN_EBREAKDOWN;
+      break;
+    }
+    if (own) {
+      x = fma(alpha, p[mine], x);
+      r = fma(-alpha, q[tid], r);
+    }
+    rz_prev = rz;
+    precondition(r, r * r, rr, rz);
+    ++it;
+    if (!isfinite(rr)) {
+      status = WN_EBREAKDOWN;
+      break;
+    }
+    if (rr <= tol2) break;
+    if (it >= A.max_iter) {
+      status = WN_ENOCONV;
+      break;
+    }
+  }
+  if (own) A.x[mine] = x;
+  if (rank == 0 && tid == 0) {
+    PcgScalars* S = A.S;
+    S->rz[0] = rz;
+    S->rz[1] = rz_prev;
+    S->bnorm2 = bb;
+    S->tol2 = tol2;
+    S->rr = rr;
+    S->alpha = alpha;
+    S->iters = it;
+    S->status = status;
+    S->max_iter = A.max_iter;
+    S->done = 1;
+  }
+  c.sync();  // no CTA leaves while another may still store into its shared memory
+}
+
+// The plan of k_small_diag from the row pointer: the row tiles of the streamed fine matrix (a row over
+// a tile's capacity, which the streamed kernels leave alone, by itself) in units, shared out evenly.
+struct SmallPlan {
+  std::vector<int4> table;
+  int tiles = 0, rows_max = 0, blocks_max = 0, units_max = 0;
+};
+SmallPlan small_plan(const int32_t* rp, int64_t n_nodes) {
+  SmallPlan P;
+  std::vector<int4> units;
+  for (int64_t r = 0; r < n_nodes; ++P.tiles) {
+    const int64_t r0 = r++;
+    while (r < n_nodes && r - r0 < kStreamRowCap && rp[r + 1] - rp[r0] <= kStreamCap) ++r;
+    for (int w = 0; w < 8 && r0 + 4 * w < r; ++w) units.push_back({(int)(r0 + 4 * w), (int)r, w, P.tiles});
+  }
+  const int slots = (P.tiles + 31) / 32 * 32;
+  const int64_t n = (int64_t)units.size();
+  for (int k = 0; k < kCtas; ++k) {
+    const int u0 = (int)(n * k / kCtas), u1 = (int)(n * (k + 1) / kCtas);
+    int lo = 0, hi = 0;
+    for (int u = u0; u < u1; ++u) {
+      const int4& t = units[u];
+      if (u == u0) lo = t.x;
+      hi = std::max(hi, std::min(t.y, t.x + 4));
+      if (t.y > t.x + 32) hi = t.y;  // rows of a further pass over the tile
+    }
+    P.table.push_back({u0, u1, lo, hi});
+    P.rows_max = std::max(P.rows_max, hi - lo);
+    P.blocks_max = std::max(P.blocks_max, rp[hi] - rp[lo]);
+    P.units_max = std::max(P.units_max, u1 - u0);
+  }
+  for (int4& u : units) u = {u.x, u.y, u.z * slots + u.w, 0};
+  P.table.insert(P.table.end(), units.begin(), units.end());
+  return P;
+}
+
+// ---------------------------------------------------------------------------------------
+// AMG with at most one level above the dense one
+// ---------------------------------------------------------------------------------------
 // first row of CTA k: multiples of 4 nodes, so that a run starts on 16 bytes in every vector
 __host__ __device__ __forceinline__ int64_t run_begin(int64_t n, int k) {
   return k >= kCtas ? n : (n * k / kCtas) & ~int64_t(3);
 }
-__host__ __device__ constexpr size_t pad16(size_t bytes) { return (bytes + 15) & ~size_t(15); }
 
 template <typename TM>
-struct SmallArgs {
+struct AmgArgs {
   int64_t n_nodes, nnzb;
   const int32_t *rp, *ci;
   const double* k64;
   const TM* km;    // the matrix in the preconditioner's precision
   const TM* dinv;  // 1 / diag
-  const TM* binv;  // block Jacobi
-  int precond, n_levels;  // n_levels: 0 (the hierarchy is its dense level) or 1
+  int n_levels;    // 0 (the hierarchy is its dense level) or 1
   TM it;                  // 1 / theta of the fine level
   const int32_t *r_rp, *r_ci, *p_rp, *p_ci;
   const TM *rv, *pv;
@@ -73,11 +408,11 @@ struct SmallArgs {
 
 // dynamic shared memory of a CTA, in this order
 template <typename TM>
-struct Layout16 {
+struct AmgLayout {
   size_t p, z, w, x, r, q, d0, cb, cx, kv, mv, ci, rp, end;
-  __host__ __device__ Layout16(int64_t n_nodes, int rows, int64_t n_coarse, int precond, int n_levels, int slice) {
+  __host__ __device__ AmgLayout(int64_t n_nodes, int rows, int64_t n_coarse, int n_levels, int slice) {
     const size_t n = 3 * (size_t)n_nodes, own = 3 * (size_t)rows, bl = (size_t)slice;
-    const bool amg = precond == 2, two = amg && n_levels > 0;
+    const bool two = n_levels > 0;
     p = 0;
     z = p + pad16(n * 8);
     w = z + pad16(n * sizeof(TM));
@@ -86,7 +421,7 @@ struct Layout16 {
     q = r + pad16(own * 8);
     d0 = q + pad16(own * 8);
     cb = d0 + (two ? pad16(own * sizeof(TM)) : 0);
-    cx = cb + (amg ? pad16((size_t)n_coarse * sizeof(TM)) : 0);
+    cx = cb + pad16((size_t)n_coarse * sizeof(TM));
     kv = cx + (two ? pad16((size_t)n_coarse * sizeof(TM)) : 0);
     mv = kv + pad16(9 * bl * 8);
     ci = mv + (two && sizeof(TM) != 8 ? pad16(9 * bl * sizeof(TM)) : 0);
@@ -96,7 +431,7 @@ struct Layout16 {
 };
 
 struct Shared {
-  double part[2][2][kCtas * kWarps];  // [dot][turn]: every warp's partial
+  double part[2][kCtas * kWarps];  // [turn]: every warp's partial
 };
 
 struct Cluster {
@@ -104,36 +439,20 @@ struct Cluster {
   Shared* sh;
   int rank, warp, lane;
   int turn = 0;
-  // this thread's contributions to N dot products, then the cluster barrier; the sums
-  template <int N>
-  __device__ __forceinline__ void dots(double (&d)[N]) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-      const double s = warp_sum(d[k]);
-      if (lane < kCtas) c.map_shared_rank(sh, lane)->part[k][turn][rank * kWarps + warp] = s;
-    }
+  // the sum of this thread's contributions to a dot product over the cluster, past its barrier
+  __device__ __forceinline__ double dot(double d) {
+    const double w = warp_sum(d);
+    if (lane < kCtas) c.map_shared_rank(sh, lane)->part[turn][rank * kWarps + warp] = w;
     c.sync();
+    double s = 0.0;
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      double s = 0.0;
-#pragma unroll
-      for (int i = 0; i < kCtas * kWarps / 32; ++i) s += sh->part[k][turn][i * 32 + lane];
-      d[k] = warp_sum(s);
-    }
+    for (int i = 0; i < kCtas * kWarps / 32; ++i) s += sh->part[turn][i * 32 + lane];
     turn ^= 1;  // the next partials go elsewhere: a slow warp may still be adding these
+    return warp_sum(s);
   }
-  // the CTA's own run [i0, i1) of a vector into the other CTAs' copies (visible after the next barrier)
   template <typename T>
   __device__ __forceinline__ void publish(T* v, int64_t i0, int64_t i1) const {
-    __syncthreads();  // the run is complete
-    const int64_t u0 = i0 * sizeof(T) / 16, u1 = (i1 * sizeof(T) + 15) / 16;
-    const int n = (int)(u1 - u0);
-    uint4* own = reinterpret_cast<uint4*>(v) + u0;
-    for (int k = threadIdx.x; k < n * (kCtas - 1); k += kThreads) {
-      const int peer = k / n, at = k - peer * n;
-      uint4* there = c.map_shared_rank(own, peer + (peer >= rank));
-      there[at] = own[at];
-    }
+    publish_run<kThreads>(c, rank, v, i0, i1);
   }
 };
 
@@ -190,7 +509,7 @@ __device__ __forceinline__ void fine_rows(const Slice<T>& M, const T* x, const E
 
 template <typename TM, bool kSlice>
 __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
-    k_small_pcg(const __grid_constant__ SmallArgs<TM> A) {
+    k_small_amg(const __grid_constant__ AmgArgs<TM> A) {
   constexpr bool kSame = std::is_same<TM, double>::value;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ Shared sh;
@@ -199,7 +518,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
   C.rank = (int)C.c.block_rank();
   const int64_t c0 = run_begin(A.n_nodes, C.rank), c1 = run_begin(A.n_nodes, C.rank + 1);
   const int64_t i0 = 3 * c0, i1 = 3 * c1, n = 3 * A.n_nodes;
-  const Layout16<TM> lay(A.n_nodes, A.rows_max, A.n_coarse, A.precond, A.n_levels, kSlice ? A.slice_blocks : 0);
+  const AmgLayout<TM> lay(A.n_nodes, A.rows_max, A.n_coarse, A.n_levels, kSlice ? A.slice_blocks : 0);
   auto at = [&](size_t off, auto tag) { return reinterpret_cast<decltype(tag)>(smem + off); };
   double* const p = at(lay.p, (double*)nullptr);   // search direction, all DOFs
   TM* const z = at(lay.z, (TM*)nullptr);           // M^-1 r, all DOFs (two-level: the residual before)
@@ -210,7 +529,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
   TM* const d0 = at(lay.d0, (TM*)nullptr) - i0;
   TM* const cb = at(lay.cb, (TM*)nullptr);
   TM* const cx = at(lay.cx, (TM*)nullptr);
-  const bool two_level = A.precond == 2 && A.n_levels > 0;
+  const bool two_level = A.n_levels > 0;
   const int gl = threadIdx.x % kLanes;
 
   // the CTA's run of the fine matrix
@@ -244,31 +563,6 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
   auto own_dofs = [&](auto f) {
     for (int64_t row = c0 + threadIdx.x / kLanes; row < c1; row += kGroups)
       if (gl < 3) f(row * 3 + gl);
-  };
-  // point / block Jacobi or none: z of the own rows, with this thread's part of r . z
-  auto diagonal = [&](double& dot) {
-    for (int64_t base = c0; base < c1; base += kGroups) {  // uniform: the shuffles need the warp
-      const int64_t row = base + threadIdx.x / kLanes;
-      const bool own = row < c1 && gl < 3;
-      const int64_t i = row * 3 + gl;
-      const TM ri = own ? (TM)r[i] : TM(0);
-      TM zi = ri;
-      if (A.precond == 3) {
-        zi = TM(0);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const TM rj = __shfl_sync(0xffffffffu, ri, j, kLanes);
-          if (own) zi = fma(__ldg(A.binv + row * 9 + gl * 3 + j), rj, zi);
-        }
-      } else if (A.precond == 1 && own) {
-        zi = __ldg(A.dinv + i) * ri;
-      }
-      if (own) {
-        z[i] = zi;
-        dot += (double)ri * (double)zi;
-      }
-    }
-    C.publish(z, i0, i1);
   };
   // the V-cycle's input of the own rows: the first smoothing step's x, or r itself
   auto vcycle_input = [&]() {
@@ -374,22 +668,18 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
   };
 
   C.c.sync();  // every CTA of the cluster has started; the run and p are in place
-  // x = 0, r = b, ||b||, z = M^-1 r
-  double d2[2] = {0.0, 0.0};
+  // x = 0, r = b, ||b||
+  double d = 0.0;
   own_dofs([&](int64_t i) {
     const double bi = __ldg(A.b + i);
     x[i] = 0.0;
     r[i] = bi;
-    d2[0] += bi * bi;
+    d += bi * bi;
   });
   __syncthreads();
-  if (A.precond == 2)
-    vcycle_input();
-  else
-    diagonal(d2[1]);
-  C.dots(d2);
-  const double bb = d2[0], tol2 = A.rtol * A.rtol * bb;
-  double rr = bb, rz = d2[1], rz_prev = 0.0, alpha = 0.0;
+  vcycle_input();
+  const double bb = C.dot(d), tol2 = A.rtol * A.rtol * bb;
+  double rr = bb, rz = 0.0, rz_prev = 0.0, alpha = 0.0;
   int it = 0, status = 0;
   bool done = false;
   if (bb == 0.0 || !isfinite(bb)) {
@@ -397,46 +687,34 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
     status = isfinite(bb) ? 0 : WN_EBREAKDOWN;
   }
   while (!done) {
-    if (A.precond == 2) {
-      double d[1] = {0.0};
-      vcycle(d[0]);
-      C.dots(d);
-      rz_prev = rz;
-      rz = d[0];
-    }
+    d = 0.0;
+    vcycle(d);
+    rz_prev = rz;
+    rz = C.dot(d);
     const double beta = it == 0 ? 0.0 : rz / rz_prev;
     for (int64_t i = threadIdx.x; i < n; i += kThreads) p[i] = fma(beta, p[i], (double)z[i]);
     __syncthreads();
-    double d[1] = {0.0};
+    d = 0.0;
     fine_rows<double>(K, p, [&](int64_t i, double t) {
       q[i] = t;
-      d[0] += p[i] * t;
+      d += p[i] * t;
     });
-    C.dots(d);
-    const double gamma = d[0];
+    const double gamma = C.dot(d);
     alpha = rz / gamma;
     if (!(gamma > 0.0) || !isfinite(alpha)) {
       status = WN_EBREAKDOWN;
       break;
     }
-    d2[0] = d2[1] = 0.0;
+    d = 0.0;
     own_dofs([&](int64_t i) {
       x[i] = fma(alpha, p[i], x[i]);
       const double ri = fma(-alpha, q[i], r[i]);
       r[i] = ri;
-      d2[0] += ri * ri;
+      d += ri * ri;
     });
     __syncwarp();
-    if (A.precond == 2)
-      vcycle_input();
-    else
-      diagonal(d2[1]);
-    C.dots(d2);
-    rr = d2[0];
-    if (A.precond != 2) {
-      rz_prev = rz;
-      rz = d2[1];
-    }
+    vcycle_input();
+    rr = C.dot(d);
     ++it;
     if (!isfinite(rr)) {
       status = WN_EBREAKDOWN;
@@ -472,10 +750,12 @@ double mat_bytes(const DevBsr& M, int value) {
 }  // namespace
 
 // The sizes at which the cluster wins (launched kernels -> cluster, us per iteration, FP64):
-//   none / point / block Jacobi   153 nodes 14.7 -> 4.8, 1,025 14.6 -> 7.4, 2,009 15.8 -> 12.5, 2,597 15.8 -> 15.9;
-//   two-level V-cycle   625 nodes 34 -> 23, 1,025 34 -> 29 with the matrix blocks in shared memory, 1,325
-//   35 -> 39 without, so there only while they fit; a dense level alone (500 nodes at most) 260 -> 90
-//   us per solve.
+//   point Jacobi   153 nodes 13.2 -> 3.9, 1,025 14.2 -> 7.0, 1,325 14.4 -> 7.6, 2,025 15.6 -> 12.7 (block Jacobi
+//   0.4 more, none the same); beyond, a thread has more than one DOF, and at 2,597 nodes an earlier
+//   form was level with the launched kernels;
+//   two-level V-cycle   625 nodes 34 -> 20, 1,025 34 -> 27.5 with the matrix blocks in shared memory, 1,325
+//   35 -> 39 without, so there only while they fit; a dense level alone (153 nodes) 250 -> 87 us per
+//   solve.
 static bool small_system(const Solid* s, const SolverWork& W, int precond) {
   if (s->bs != 3 || s->n_nodes > kMaxNodes || W.profile || W.half) return false;
   // (the failure hook and shortened waits of the streamed kernels are theirs to report)
@@ -483,12 +763,75 @@ static bool small_system(const Solid* s, const SolverWork& W, int precond) {
   return precond != 2 || s->amg->levels.empty() || (s->amg->degree == 1 && s->amg->levels.size() == 1);
 }
 
+// a kernel of one cluster (an error where 16 SMs of a GPC are not to be had)
+template <typename ARGS>
+static cudaError_t launch_cluster(void (*kern)(ARGS), const ARGS& A, int threads, size_t smem, size_t limit,
+                                  cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+  if (e != cudaSuccess) return e;
+  kern<<<kCtas, threads, smem, st>>>(A);
+  return cudaGetLastError();
+}
+
+// none / Jacobi / block Jacobi: 0 with the kernel under way, 1 for the launched kernels
 template <typename TM>
-int small_pcg(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, int precond, PcgScalars* S,
-              cudaStream_t st, PcgScalars* hS) {
-  if (!small_system(s, W, precond)) return 1;
+static int start_diag(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, int precond,
+                      PcgScalars* S, cudaStream_t st) {
+  if (W.small_tiles == 0) {  // the pattern's plan, kept with the workspace
+    const SmallPlan P = small_plan(s->h_row_ptr.data(), s->n_nodes);
+    WN_CHECK(W.small_plan.upload(P.table));
+    WN_CUDA(cudaStreamSynchronize(0));
+    W.small_tiles = P.tiles;
+    W.small_rows = P.rows_max;
+    W.small_blocks = P.blocks_max;
+    W.small_units = P.units_max;
+  }
+  if (W.small_tiles > kMaxTiles) return 1;
+  DiagArgs<TM> A{};
+  A.n_nodes = s->n_nodes;
+  A.nnzb = s->nnzb;
+  A.rp = s->row_ptr.p;
+  A.ci = s->col_idx.p;
+  A.k64 = s->k64.p;
+  if constexpr (std::is_same<TM, double>::value) {
+    A.dinv = W.dinv64.p;
+    A.binv = W.binv64.p;
+  } else {
+    A.dinv = W.dinv32.p;
+    A.binv = W.binv32.p;
+  }
+  A.precond = precond;
+  A.b = b;
+  A.x = W.p64.x.p;
+  A.plan = W.small_plan.p;
+  A.slots = (W.small_tiles + 31) / 32 * 32;
+  for (int k = 0; k < kCtas; ++k)
+    A.own_max = std::max(A.own_max, 32 * (int)(own_begin(s->n_nodes, k + 1) - own_begin(s->n_nodes, k)));
+  A.rows_max = W.small_rows;
+  A.units_max = W.small_units;
+  A.rtol = rtol;
+  A.max_iter = max_iter;
+  A.S = S;
+  auto bytes = [&](int held) { return DiagLayout<TM>(A.n_nodes, A.slots, A.own_max, A.rows_max, A.units_max, held).end; };
+  constexpr int kBlockBytes = 9 * 8 + 4;
+  if (bytes(0) + 32 > kDiagSmemLimit) return 1;  // (two roundings to 16 bytes)
+  A.slice_blocks = std::min<int>(W.small_blocks, (int)((kDiagSmemLimit - 32 - bytes(0)) / kBlockBytes));
+  const size_t smem = bytes(A.slice_blocks);
+  const cudaError_t e =
+      A.slice_blocks == W.small_blocks
+          ? launch_cluster(k_small_diag<TM, true>, A, kDiagThreads, smem, kDiagSmemLimit, st)
+          : launch_cluster(k_small_diag<TM, false>, A, kDiagThreads, smem, kDiagSmemLimit, st);
+  return e == cudaSuccess ? 0 : 1;
+}
+
+// AMG with at most one level above the dense one: 0 with the kernel under way, 1 for the launched kernels
+template <typename TM>
+static int start_amg(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, PcgScalars* S,
+                     cudaStream_t st) {
   constexpr bool kSame = std::is_same<TM, double>::value;
-  SmallArgs<TM> A{};
+  AmgHierarchy& H = *s->amg;
+  AmgArgs<TM> A{};
   A.n_nodes = s->n_nodes;
   A.nnzb = s->nnzb;
   A.rp = s->row_ptr.p;
@@ -499,37 +842,26 @@ int small_pcg(Solid* s, SolverWork& W, const double* b, double rtol, int max_ite
   if constexpr (kSame) {
     A.km = s->k64.p;
     A.dinv = W.dinv64.p;
-    A.binv = W.binv64.p;
   } else {
     A.km = s->k32.p;
     A.dinv = W.dinv32.p;
-    A.binv = W.binv32.p;
   }
-  A.precond = precond;
-  const double n = (double)W.n, nK = 8.0 * n, nM = n * sizeof(TM);
-  double prec_bytes = (precond == 1 ? 3.0 : precond == 3 ? 5.0 : 2.0) * nM;
-  if (precond == 2) {
-    AmgHierarchy& H = *s->amg;
-    A.n_levels = (int)H.levels.size();
-    A.n_coarse = H.n_coarse;
-    A.coarse_inv = H.coarse_inv.p;
-    prec_bytes = 8.0 * (double)H.n_coarse * (double)H.n_coarse + 2.0 * (double)H.n_coarse * sizeof(TM);
-    if (A.n_levels > 0) {
-      DevLevel& L = H.levels[0];
-      A.it = (TM)L.inv_theta;
-      A.r_rp = L.R.rp.p;
-      A.r_ci = L.R.ci.p;
-      A.p_rp = L.P.rp.p;
-      A.p_ci = L.P.ci.p;
-      if constexpr (kSame) {
-        A.rv = L.R.v64.p;
-        A.pv = L.P.v64.p;
-      } else {
-        A.rv = L.R.v32.p;
-        A.pv = L.P.v32.p;
-      }
-      const double fine = (double)s->nnzb * (9 * sizeof(TM) + 4) + 4.0 * (double)(s->n_nodes + 1);
-      prec_bytes += 2.0 * fine + mat_bytes(L.P, sizeof(TM)) + mat_bytes(L.R, sizeof(TM)) + 11.0 * nM;
+  A.n_levels = (int)H.levels.size();
+  A.n_coarse = H.n_coarse;
+  A.coarse_inv = H.coarse_inv.p;
+  if (A.n_levels > 0) {
+    DevLevel& L = H.levels[0];
+    A.it = (TM)L.inv_theta;
+    A.r_rp = L.R.rp.p;
+    A.r_ci = L.R.ci.p;
+    A.p_rp = L.P.rp.p;
+    A.p_ci = L.P.ci.p;
+    if constexpr (kSame) {
+      A.rv = L.R.v64.p;
+      A.pv = L.P.v64.p;
+    } else {
+      A.rv = L.R.v32.p;
+      A.pv = L.P.v32.p;
     }
   }
   A.rtol = rtol;
@@ -543,33 +875,43 @@ int small_pcg(Solid* s, SolverWork& W, const double* b, double rtol, int max_ite
   }
   A.rows_max = (int)rows;
   A.slice_blocks = (int)blocks;
-  auto bytes = [&](int slice) {
-    return Layout16<TM>(A.n_nodes, A.rows_max, A.n_coarse, precond, A.n_levels, slice).end;
-  };
+  auto bytes = [&](int slice) { return AmgLayout<TM>(A.n_nodes, A.rows_max, A.n_coarse, A.n_levels, slice).end; };
   const bool slice = bytes(A.slice_blocks) <= kSmemLimit;
   if (!slice && A.n_levels > 0) return 1;
   const size_t smem = bytes(slice ? A.slice_blocks : 0);
   if (smem > kSmemLimit) return 1;
-  auto launch = [&](auto kern) -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
-    if (e != cudaSuccess) return e;
-    kern<<<kCtas, kThreads, smem, st>>>(A);
-    return cudaGetLastError();
-  };
-  if ((slice ? launch(k_small_pcg<TM, true>) : launch(k_small_pcg<TM, false>)) != cudaSuccess) {
+  const cudaError_t e = slice ? launch_cluster(k_small_amg<TM, true>, A, kThreads, smem, kSmemLimit, st)
+                              : launch_cluster(k_small_amg<TM, false>, A, kThreads, smem, kSmemLimit, st);
+  return e == cudaSuccess ? 0 : 1;
+}
+
+template <typename TM>
+int small_pcg(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, int precond, PcgScalars* S,
+              cudaStream_t st, PcgScalars* hS) {
+  if (!small_system(s, W, precond)) return 1;
+  const int rc = precond == 2 ? start_amg<TM>(s, W, b, rtol, max_iter, S, st)
+                              : start_diag<TM>(s, W, b, rtol, max_iter, precond, S, st);
+  if (rc != 0) {
     cudaGetLastError();
-    return 1;  // no room for a cluster of 16 here: the launched kernels
+    return rc;  // 1: too many tiles, or no room for a cluster of 16 here
   }
   W.launches++;
   WN_CUDA(cudaMemcpyAsync(hS, S, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
   WN_CUDA(cudaStreamSynchronize(st));
-  // Out of iterations, hundreds from convergence: such an iterate depends on the order of the dot
-  // products, so it is left to the launched kernels, whose order does not depend on this rule.
-  if (hS->status == WN_ENOCONV && precond != 2) return 1;
   // algorithmic bytes as the launched kernels count them: I products and updates, I preconditioner
   // applies (the first before the iterations, none after the last)
-  const double fine64 = (double)s->nnzb * 76.0 + 4.0 * (double)(s->n_nodes + 1);
+  const double n = (double)W.n, nK = 8.0 * n, nM = n * sizeof(TM);
+  const double rows = 4.0 * (double)(s->n_nodes + 1);
+  double prec_bytes = (precond == 1 ? 3.0 : precond == 3 ? 5.0 : 2.0) * nM;
+  if (precond == 2) {
+    const AmgHierarchy& H = *s->amg;
+    const double nc = (double)H.n_coarse;
+    prec_bytes = 8.0 * nc * nc + 2.0 * nc * sizeof(TM);
+    if (!H.levels.empty())
+      prec_bytes += 2.0 * ((double)s->nnzb * (9 * sizeof(TM) + 4) + rows) + mat_bytes(H.levels[0].P, sizeof(TM)) +
+                    mat_bytes(H.levels[0].R, sizeof(TM)) + 11.0 * nM;
+  }
+  const double fine64 = (double)s->nnzb * 76.0 + rows;
   W.bytes += 3.0 * nK + hS->iters * (fine64 + nM + 9.0 * nK) + std::max(1, hS->iters) * prec_bytes;
   return 0;
 }

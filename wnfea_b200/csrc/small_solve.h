@@ -9,8 +9,8 @@
 namespace wn {
 
 // Solves K x = b from x = 0 to ||r|| <= rtol ||b|| (x in W.p64.x) with the preconditioner in TM and
-// copies the result's scalars to hS.  0: done; 1: for the launched kernels (not a small system, no
-// room for the cluster, or point Jacobi out of iterations); anything else: an error.
+// copies the result's scalars to hS.  0: done; 1: for the launched kernels (not a small system, or no
+// room for the cluster); anything else: an error.
 template <typename TM>
 int small_pcg(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, int precond, PcgScalars* S,
               cudaStream_t st, PcgScalars* hS);
