@@ -7,6 +7,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
+from wnfea_b200.amg import AMGParams
 from wnfea_b200.mesh import generate_c3d10_kuhn_block, tip_load_cases
 from wnfea_b200.model import solid_fixed_dofs
 from wnfea_b200.solid_solver import assemble_c3d10_sparse_3dof
@@ -53,3 +54,32 @@ def test_iteration_limit_returns_the_iterate_once(cells, limit, precond):
     assert st["kernel_launches"] < 20
     st = s.solve(F, rtol=1e-6, max_iter=limit, precond=precond, precision=1)[1]
     assert st["status"] == -5 and st["iterations"] == limit and st["kernel_launches"] < 20
+
+
+# a launch runs 2,048 iterations at most (128 with AMG), whatever the caller's limit, and the next goes on
+# with the same bits
+@pytest.mark.parametrize("cells", [(37, 1, 1), (34, 2, 1)])
+@pytest.mark.parametrize("precond", [0, 1, 3])
+def test_long_solves_take_several_launches(cells, precond):
+    s, F = _system(*cells, seed=11)
+    kw = dict(rtol=1e-30, precond=precond, max_outer=1)
+    launches = [s.solve(F, max_iter=n, **kw)[1]["kernel_launches"] for n in (2048, 2049)]
+    assert launches[1] == launches[0] + 1
+    st = _same(s, F, max_iter=5000, **kw)
+    # (a Jacobi solve's recurrence may reach 1e-30 within one launch more)
+    assert st["iterations"] > 2048 and st["kernel_launches"] >= launches[1]
+
+
+# (sizes whose matrix copies fit shared memory)
+@pytest.mark.parametrize("cells,precision", [((20, 2, 2), 0), ((12, 2, 2), 1)])
+def test_long_amg_solve_takes_several_launches(cells, precision):
+    s, F = _system(*cells, seed=13)
+    s.amg_setup(AMGParams(cheb_safety=1e6))  # hardly any smoothing: some hundred iterations
+    u, st = s.solve(F, rtol=1e-13, precond=2, precision=precision, max_outer=1)
+    v, sv = s.solve(F, rtol=1e-13, precond=2, precision=precision, max_outer=1, profile=True)
+    few = s.solve(F, rtol=1e-2, precond=2, precision=precision, max_outer=1)[1]
+    assert st["iterations"] > 128 >= few["iterations"]
+    assert st["kernel_launches"] == few["kernel_launches"] + (st["iterations"] - 1) // 128
+    # the launched kernels' sums run in another order; a lost direction would cost a start from scratch
+    assert abs(st["iterations"] - sv["iterations"]) <= 0.05 * sv["iterations"]
+    assert np.linalg.norm(u - v) <= 1e-9 * np.linalg.norm(v)

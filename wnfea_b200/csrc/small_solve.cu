@@ -46,6 +46,10 @@ constexpr int kLanes = 8;                   // lanes per block row
 constexpr int kGroups = kThreads / kLanes;  // rows of a CTA side by side
 constexpr int kTeam = 4, kTeams = kWarps / kTeam;  // warps per row of the restriction
 constexpr int64_t kMaxNodes = 2048;         // (small_system)
+// Iterations of one launch (8 to 26 ms; 4 ms with AMG, whose solves take some 40): the caller's max_iter
+// bounds a solve, not the length of a kernel.  The next launch goes on from x, r, p and the scalars in
+// global memory, with the same bits.
+constexpr int kDiagSteps = 2048, kAmgSteps = 128;
 constexpr size_t kSmemLimit = 214 * 1024;   // dynamic shared memory (5 KB are static)
 
 __host__ __device__ constexpr size_t pad16(size_t bytes) { return (bytes + 15) & ~size_t(15); }
@@ -94,7 +98,8 @@ struct DiagArgs {
   const TM* binv;  // block Jacobi
   int precond;
   const double* b;
-  double* x;
+  double *x, *r, *p;  // r, p: the state between launches
+  int first;          // from x = 0, or on from the state
   const int4* plan;  // kCtas runs (first unit, end, first row, end), then the units (small_plan)
   int slots;         // tiles rounded up to 32
   int own_max, rows_max, units_max;
@@ -175,7 +180,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kDiagThreads, 1)
     for (int k = 0; k < 9; ++k) sk[k * A.slice_blocks + b] = __ldg(A.k64 + k * A.nnzb + q0 + far + b);
   }
   const TM di = A.precond == 1 && own ? __ldg(A.dinv + mine) : TM(1);
-  for (int64_t i = tid; i < n; i += kDiagThreads) p[i] = 0.0;
+  for (int64_t i = tid; i < n; i += kDiagThreads) p[i] = A.first ? 0.0 : A.p[i];
   for (int i = tid; i < 8 * A.slots; i += kDiagThreads) pq[i] = 0.0;  // units and warps without rows add zero
   for (int i = tid; i < 8 * 32; i += kDiagThreads) srr[i] = srz[i] = 0.0;
 
@@ -287,12 +292,13 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kDiagThreads, 1)
   };
 
   c.sync();  // every CTA of the cluster has started; its zeros are in place
-  double x = 0.0, r = own ? __ldg(A.b + mine) : 0.0, bb, rz;
-  precondition(r, r * r, bb, rz);
-  const double tol2 = A.rtol * A.rtol * bb;
-  double rr = bb, rz_prev = 0.0, alpha = 0.0;
-  int it = 0, status = 0;
-  bool done = false;
+  double x = own && !A.first ? A.x[mine] : 0.0, r = own ? (A.first ? A.b[mine] : A.r[mine]) : 0.0, rr, rz;
+  precondition(r, r * r, rr, rz);
+  const double bb = A.first ? rr : A.S->bnorm2, tol2 = A.rtol * A.rtol * bb;
+  double rz_prev = A.first ? 0.0 : A.S->rz[1], alpha = 0.0;
+  const int it0 = A.first ? 0 : A.S->iters;
+  int it = it0, status = 0;
+  bool done = false, running = false;
   if (bb == 0.0 || !isfinite(bb)) {
     done = true;
     status = isfinite(bb) ? 0 : WN_EBREAKDOWN;
@@ -323,8 +329,16 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kDiagThreads, 1)
       status = WN_ENOCONV;
       break;
     }
+    if (it - it0 >= kDiagSteps) {
+      running = true;
+      break;
+    }
   }
   if (own) A.x[mine] = x;
+  if (own && running) {
+    A.r[mine] = r;
+    A.p[mine] = p[mine];
+  }
   if (rank == 0 && tid == 0) {
     PcgScalars* S = A.S;
     S->rz[0] = rz;
@@ -336,7 +350,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kDiagThreads, 1)
     S->iters = it;
     S->status = status;
     S->max_iter = A.max_iter;
-    S->done = 1;
+    S->done = !running;
   }
   c.sync();  // no CTA leaves while another may still store into its shared memory
 }
@@ -398,7 +412,8 @@ struct AmgArgs {
   int64_t n_coarse;
   const double* coarse_inv;
   const double* b;
-  double* x;
+  double *x, *r, *p;  // r, p: the state between launches
+  int first;          // from x = 0, or on from the state
   int slice_blocks;  // blocks of the longest run in shared memory, 0: read from L2
   int rows_max;
   double rtol;
@@ -557,7 +572,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
     else
       M = {sm, sc, sr, A.slice_blocks, c0, c1};
   }
-  for (int64_t i = threadIdx.x; i < n; i += kThreads) p[i] = 0.0;
+  for (int64_t i = threadIdx.x; i < n; i += kThreads) p[i] = A.first ? 0.0 : A.p[i];
 
   // f(i) for the DOFs of the CTA's rows, by the lanes that own them in fine_rows
   auto own_dofs = [&](auto f) {
@@ -671,17 +686,19 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
   // x = 0, r = b, ||b||
   double d = 0.0;
   own_dofs([&](int64_t i) {
-    const double bi = __ldg(A.b + i);
-    x[i] = 0.0;
-    r[i] = bi;
-    d += bi * bi;
+    const double ri = A.first ? A.b[i] : A.r[i];
+    x[i] = A.first ? 0.0 : A.x[i];
+    r[i] = ri;
+    d += ri * ri;
   });
   __syncthreads();
   vcycle_input();
-  const double bb = C.dot(d), tol2 = A.rtol * A.rtol * bb;
-  double rr = bb, rz = 0.0, rz_prev = 0.0, alpha = 0.0;
-  int it = 0, status = 0;
-  bool done = false;
+  double rr = C.dot(d);
+  const double bb = A.first ? rr : A.S->bnorm2, tol2 = A.rtol * A.rtol * bb;
+  double rz = A.first ? 0.0 : A.S->rz[0], rz_prev = 0.0, alpha = 0.0;
+  const int it0 = A.first ? 0 : A.S->iters;
+  int it = it0, status = 0;
+  bool done = false, running = false;
   if (bb == 0.0 || !isfinite(bb)) {
     done = true;
     status = isfinite(bb) ? 0 : WN_EBREAKDOWN;
@@ -725,8 +742,18 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
       status = WN_ENOCONV;
       break;
     }
+    if (it - it0 >= kAmgSteps) {
+      running = true;
+      break;
+    }
   }
-  own_dofs([&](int64_t i) { A.x[i] = x[i]; });
+  own_dofs([&](int64_t i) {
+    A.x[i] = x[i];
+    if (running) {
+      A.r[i] = r[i];
+      A.p[i] = p[i];
+    }
+  });
   if (C.rank == 0 && threadIdx.x == 0) {
     PcgScalars* S = A.S;
     S->rz[0] = rz;
@@ -738,7 +765,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
     S->iters = it;
     S->status = status;
     S->max_iter = A.max_iter;
-    S->done = 1;
+    S->done = !running;
   }
   C.c.sync();  // no CTA leaves while another may still store into its shared memory
 }
@@ -776,7 +803,7 @@ static cudaError_t launch_cluster(void (*kern)(ARGS), const ARGS& A, int threads
 
 // none / Jacobi / block Jacobi: 0 with the kernel under way, 1 for the launched kernels
 template <typename TM>
-static int start_diag(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, int precond,
+static int start_diag(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, int precond, bool first,
                       PcgScalars* S, cudaStream_t st) {
   if (W.small_tiles == 0) {  // the pattern's plan, kept with the workspace
     const SmallPlan P = small_plan(s->h_row_ptr.data(), s->n_nodes);
@@ -804,6 +831,9 @@ static int start_diag(Solid* s, SolverWork& W, const double* b, double rtol, int
   A.precond = precond;
   A.b = b;
   A.x = W.p64.x.p;
+  A.r = W.p64.r.p;
+  A.p = W.p64.p0.p;
+  A.first = first;
   A.plan = W.small_plan.p;
   A.slots = (W.small_tiles + 31) / 32 * 32;
   for (int k = 0; k < kCtas; ++k)
@@ -827,8 +857,8 @@ static int start_diag(Solid* s, SolverWork& W, const double* b, double rtol, int
 
 // AMG with at most one level above the dense one: 0 with the kernel under way, 1 for the launched kernels
 template <typename TM>
-static int start_amg(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, PcgScalars* S,
-                     cudaStream_t st) {
+static int start_amg(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, bool first,
+                     PcgScalars* S, cudaStream_t st) {
   constexpr bool kSame = std::is_same<TM, double>::value;
   AmgHierarchy& H = *s->amg;
   AmgArgs<TM> A{};
@@ -839,6 +869,9 @@ static int start_amg(Solid* s, SolverWork& W, const double* b, double rtol, int 
   A.k64 = s->k64.p;
   A.b = b;
   A.x = W.p64.x.p;
+  A.r = W.p64.r.p;
+  A.p = W.p64.p0.p;
+  A.first = first;
   if constexpr (kSame) {
     A.km = s->k64.p;
     A.dinv = W.dinv64.p;
@@ -889,15 +922,18 @@ template <typename TM>
 int small_pcg(Solid* s, SolverWork& W, const double* b, double rtol, int max_iter, int precond, PcgScalars* S,
               cudaStream_t st, PcgScalars* hS) {
   if (!small_system(s, W, precond)) return 1;
-  const int rc = precond == 2 ? start_amg<TM>(s, W, b, rtol, max_iter, S, st)
-                              : start_diag<TM>(s, W, b, rtol, max_iter, precond, S, st);
-  if (rc != 0) {
-    cudaGetLastError();
-    return rc;  // 1: too many tiles, or no room for a cluster of 16 here
+  hS->done = 0;
+  for (bool first = true; !hS->done; first = false) {
+    const int rc = precond == 2 ? start_amg<TM>(s, W, b, rtol, max_iter, first, S, st)
+                                : start_diag<TM>(s, W, b, rtol, max_iter, precond, first, S, st);
+    if (rc != 0) {
+      cudaGetLastError();
+      return rc;  // 1: too many tiles, or no room for a cluster of 16 here
+    }
+    W.launches++;
+    WN_CUDA(cudaMemcpyAsync(hS, S, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
+    WN_CUDA(cudaStreamSynchronize(st));
   }
-  W.launches++;
-  WN_CUDA(cudaMemcpyAsync(hS, S, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
-  WN_CUDA(cudaStreamSynchronize(st));
   // algorithmic bytes as the launched kernels count them: I products and updates, I preconditioner
   // applies (the first before the iterations, none after the last)
   const double n = (double)W.n, nK = 8.0 * n, nM = n * sizeof(TM);
