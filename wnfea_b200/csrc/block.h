@@ -40,23 +40,60 @@ struct BlockScalarsT {
   int max_iter;
 };
 
+// The device vectors of the batched solves of one handle, shared by the batch widths: one batch runs
+// at a time and leaves nothing in them for the next, so each vector is kept once, as long as the widest
+// batch so far needs it, and a narrower one uses its beginning.  (A workspace per width held 56
+// columns after a load book of 32, one of 16 and one of 5 cases.)
+struct BatchStore {
+  std::vector<DArray<unsigned char>> vecs;
+  uint64_t epoch = 0;         // changes whenever a vector moves: captured graphs hold the addresses
+  uint64_t hierarchy_id = 0;  // the AmgHierarchy that the level vectors were sized for
+  int at_least(int id, int64_t bytes) {
+    if ((size_t)id >= vecs.size()) vecs.resize(id + 1);
+    if (vecs[id].n >= bytes) return 0;
+    ++epoch;
+    return vecs[id].alloc(bytes);
+  }
+  void release_from(int id) {
+    ++epoch;
+    if ((size_t)id < vecs.size()) vecs.resize(id);
+  }
+};
+enum BatchVecId {
+  kVecPartA, kVecPartB, kVecPartC, kVecF, kVecU, kVecUlo, kVecR, kVecX, kVecRes, kVecP0, kVecP1, kVecQ, kVecDinv64,
+  kVecDinv32, kVecZ32, kVecR32, kVecD32, kVecZ64, kVecD64,
+  kVecHierarchy,  // from here on sized for the hierarchy: the coarsest level's four, then 7 per level and precision
+  kVecCb32 = kVecHierarchy, kVecCx32, kVecCb64, kVecCx64, kVecLevels
+};
+template <typename T>
+struct BatchVec {
+  T* p = nullptr;
+  int take(BatchStore& M, int id, int64_t n) {
+    p = nullptr;
+    WN_CHECK(M.at_least(id, n * (int64_t)sizeof(T)));
+    p = reinterpret_cast<T*>(M.vecs[id].p);
+    return 0;
+  }
+};
+
 // Vectors of a V-cycle level.  The finest level's right-hand side and result are the PCG's, and r, d
 // and d2 belong to Chebyshev steps beyond the first: left out where nothing reads them (at 32 cases
 // a fine vector of a million DOFs is 130 MB in FP32).
 template <typename T>
 struct BatchLevelVecs {
-  DArray<T> b, x, x2, r, d, d2, res;
-  int alloc(int64_t n, bool finest, int degree) {
-    if (!finest) {
-      WN_CHECK(b.alloc(n));
-      WN_CHECK(x2.alloc(n));
+  BatchVec<T> b, x, x2, r, d, d2, res;
+  int take(BatchStore& M, int level, int64_t n, int degree) {
+    const int id = kVecLevels + 7 * (2 * level + (sizeof(T) == 8));
+    if (level > 0) {
+      WN_CHECK(b.take(M, id, n));
+      WN_CHECK(x2.take(M, id + 1, n));
     }
-    WN_CHECK(x.alloc(n));
-    WN_CHECK(res.alloc(n));
+    WN_CHECK(x.take(M, id + 2, n));
+    WN_CHECK(res.take(M, id + 3, n));
     if (degree > 1) {
-      WN_CHECK(r.alloc(n));
-      WN_CHECK(d.alloc(n));
-      WN_CHECK(d2.alloc(n));
+      WN_CHECK(r.take(M, id + 4, n));
+      WN_CHECK(d.take(M, id + 5, n));
+      WN_CHECK(d2.take(M, id + 6, n));
     }
     return 0;
   }
@@ -67,29 +104,29 @@ struct BlockWorkT {
   int64_t n = 0;  // scalar DOFs of the fine level
   static constexpr int kMaxParts = 148 * 16;
   int npA = 0, npB = 0, npC = 0;
-  DArray<double> partA, partB, partC;  // kMaxParts x kBatch
-  DArray<BlockScalarsT<kBatch>> scal;  // [0] inner PCG, [1] outer column norms
-  DArray<double> rtol_cols;            // kBatch inner targets
+  uint64_t epoch = 0;  // the store's when the graphs were captured
+  BatchVec<double> partA, partB, partC;  // kMaxParts x kBatch
+  DArray<BlockScalarsT<kBatch>> scal;    // [0] inner PCG, [1] outer column norms
+  DArray<double> rtol_cols;              // kBatch inner targets
   std::vector<double> h_rtol;
   // outer refinement: F, U = U + Ulo (double-double), R = F - K U
-  DArray<double> F, U, Ulo, R;
+  BatchVec<double> F, U, Ulo, R;
   // Krylov vectors (FP64)
-  DArray<double> x, r, p0, p1, q;
+  BatchVec<double> x, r, p0, p1, q;
   // 1 / diag of the fine matrix (refreshed per solve)
-  DArray<double> dinv64;
-  DArray<float> dinv32;
+  BatchVec<double> dinv64;
+  BatchVec<float> dinv32;
   // preconditioner input / output in the V-cycle precision
-  DArray<float> z32, r32;
-  DArray<double> z64;
+  BatchVec<float> z32, r32;
+  BatchVec<double> z64;
   // the fine V-cycle's first smoothing input dinv r / theta, written by the PCG update
-  DArray<float> d0_32;
-  DArray<double> d0_64;
+  BatchVec<float> d0_32;
+  BatchVec<double> d0_64;
   // V-cycle vectors per level and the coarsest right-hand side / solution
   std::vector<BatchLevelVecs<float>> lv32;
   std::vector<BatchLevelVecs<double>> lv64;
-  DArray<float> cb32, cx32;
-  DArray<double> cb64, cx64;
-  uint64_t hierarchy_id = 0;        // the AmgHierarchy the level vectors were sized for
+  BatchVec<float> cb32, cx32;
+  BatchVec<double> cb64, cx64;
   // x-tiles of the fine level (block_batch.cuh build_x_tiles): runs of rows whose blocks name at
   // most 256 columns; per tile its sorted columns, per block its column's index among them
   DArray<int32_t> xt_rows, xt_col_ptr, xt_cols;
@@ -108,6 +145,7 @@ struct BlockWorkT {
 struct BlockSet {
   // the fine level's rows as the row kernels of 2 and 3 CTAs per SM take them (batch_order)
   DArray<int32_t> order[2];
+  BatchStore store;
   std::unique_ptr<BlockWorkT<8>> w8;
   std::unique_ptr<BlockWorkT<16>> w16;
   std::unique_ptr<BlockWorkT<32>> w32;

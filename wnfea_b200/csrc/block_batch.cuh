@@ -2061,72 +2061,57 @@ BlockWork* block_work(BlockSet& B) {
 
 int ensure_block_work(Solid* s, int vmode, int precond) {
   BlockWork& W = *block_work(*s->batch);
-  const int64_t n = s->n_nodes * 3;
-  const int64_t nb = n * kBatch;
-  if (W.n != n) {
-    W.n = n;
-    WN_CHECK(W.F.alloc(nb));
-    WN_CHECK(W.U.alloc(nb));
-    WN_CHECK(W.Ulo.alloc(nb));
-    WN_CHECK(W.R.alloc(nb));
-    WN_CHECK(W.x.alloc(nb));
-    WN_CHECK(W.r.alloc(nb));
-    WN_CHECK(W.q.alloc(nb));
-    WN_CHECK(W.dinv64.alloc(n));
-    WN_CHECK(W.dinv32.alloc(n));
-    for (auto& a : W.graphs)
-      for (auto& g : a) g.reset();
+  BatchStore& M = s->batch->store;
+  const int64_t n = s->n_nodes * 3, nb = n * kBatch;
+  const int64_t np = (int64_t)BlockWork::kMaxParts * kBatch;
+  if (precond == 2 && M.hierarchy_id != s->amg->id) {
+    M.release_from(kVecHierarchy);
+    M.hierarchy_id = s->amg->id;
   }
-  // search directions: one FP32 vector in place, or two FP64 ones (grown, never shrunk: the graphs of
-  // the other precision hold their addresses)
+  W.n = n;
+  WN_CHECK(W.partA.take(M, kVecPartA, np));
+  WN_CHECK(W.partB.take(M, kVecPartB, np));
+  WN_CHECK(W.partC.take(M, kVecPartC, np));
+  WN_CHECK(W.F.take(M, kVecF, nb));
+  WN_CHECK(W.U.take(M, kVecU, nb));
+  WN_CHECK(W.Ulo.take(M, kVecUlo, nb));
+  WN_CHECK(W.R.take(M, kVecR, nb));
+  WN_CHECK(W.x.take(M, kVecX, nb));
+  WN_CHECK(W.r.take(M, kVecRes, nb));
+  WN_CHECK(W.q.take(M, kVecQ, nb));
+  WN_CHECK(W.dinv64.take(M, kVecDinv64, n));
+  WN_CHECK(W.dinv32.take(M, kVecDinv32, n));
+  // search directions: one FP32 vector in place, or two FP64 ones
   const bool p32 = vmode == 1 && fp32_directions<float>(s);
-  const int64_t np0 = p32 ? (nb + 1) / 2 : nb;
-  if (W.p0.n < np0 || (!p32 && W.p1.n < nb)) {
-    for (auto& a : W.graphs)
-      for (auto& g : a) g.reset();
-    if (W.p0.n < np0) WN_CHECK(W.p0.alloc(np0));
-    if (!p32 && W.p1.n < nb) WN_CHECK(W.p1.alloc(nb));
-  }
+  WN_CHECK(W.p0.take(M, kVecP0, p32 ? (nb + 1) / 2 : nb));
+  if (!p32) WN_CHECK(W.p1.take(M, kVecP1, nb));
   if (vmode == 1) {
-    WN_CHECK(W.z32.alloc(nb));
-    WN_CHECK(W.r32.alloc(nb));
-    if (precond == 2) WN_CHECK(W.d0_32.alloc(nb));
+    WN_CHECK(W.z32.take(M, kVecZ32, nb));
+    WN_CHECK(W.r32.take(M, kVecR32, nb));
+    if (precond == 2) WN_CHECK(W.d0_32.take(M, kVecD32, nb));
   } else {
-    WN_CHECK(W.z64.alloc(nb));
-    if (precond == 2) WN_CHECK(W.d0_64.alloc(nb));
+    WN_CHECK(W.z64.take(M, kVecZ64, nb));
+    if (precond == 2) WN_CHECK(W.d0_64.take(M, kVecD64, nb));
   }
-  WN_CHECK(W.partA.alloc((int64_t)BlockWork::kMaxParts * kBatch));
-  WN_CHECK(W.partB.alloc((int64_t)BlockWork::kMaxParts * kBatch));
-  WN_CHECK(W.partC.alloc((int64_t)BlockWork::kMaxParts * kBatch));
   WN_CHECK(W.scal.alloc(2));
   WN_CHECK(W.rtol_cols.alloc(kBatch));
   W.h_rtol.assign(kBatch, 1.0);
   if (precond == 2) {
     AmgHierarchy& H = *s->amg;
-    if (W.hierarchy_id != H.id) {
-      W.lv32.clear();
-      W.lv64.clear();
-      W.cb32.release();
-      W.cx32.release();
-      W.cb64.release();
-      W.cx64.release();
-      W.hierarchy_id = H.id;
-      for (auto& a : W.graphs)
-        for (auto& g : a) g.reset();
-    }
     const size_t nl = H.levels.size();
-    if (vmode == 1 && W.lv32.size() != nl) {
-      W.lv32.resize(nl);
-      for (size_t l = 0; l < nl; ++l) WN_CHECK(W.lv32[l].alloc(H.levels[l].n_nodes * H.levels[l].bs * kBatch, l == 0, H.degree));
-      WN_CHECK(W.cb32.alloc(H.n_coarse * kBatch));
-      WN_CHECK(W.cx32.alloc(H.n_coarse * kBatch));
-    }
-    if (vmode == 0 && W.lv64.size() != nl) {
-      W.lv64.resize(nl);
-      for (size_t l = 0; l < nl; ++l) WN_CHECK(W.lv64[l].alloc(H.levels[l].n_nodes * H.levels[l].bs * kBatch, l == 0, H.degree));
-      WN_CHECK(W.cb64.alloc(H.n_coarse * kBatch));
-      WN_CHECK(W.cx64.alloc(H.n_coarse * kBatch));
-    }
+    auto levels = [&](auto& lv, auto& cb, auto& cx, int id) -> int {
+      lv.resize(nl);
+      for (size_t l = 0; l < nl; ++l)
+        WN_CHECK(lv[l].take(M, (int)l, H.levels[l].n_nodes * H.levels[l].bs * kBatch, H.degree));
+      WN_CHECK(cb.take(M, id, H.n_coarse * kBatch));
+      return cx.take(M, id + 1, H.n_coarse * kBatch);
+    };
+    WN_CHECK(vmode == 1 ? levels(W.lv32, W.cb32, W.cx32, kVecCb32) : levels(W.lv64, W.cb64, W.cx64, kVecCb64));
+  }
+  if (W.epoch != M.epoch) {  // some vector has moved since the graphs were captured
+    W.epoch = M.epoch;
+    for (auto& a : W.graphs)
+      for (auto& g : a) g.reset();
   }
   if (kBatch == 32 && s->batch_stage_x && !W.xt_tried) WN_CHECK(build_x_tiles(s, W));
   return 0;
