@@ -251,7 +251,7 @@ struct BPNew {  // p_new = z + beta p_old per case (FP64 Krylov, double case map
     const C4<double> pp = ldc<double>(p + i * kBatch, l);
     C4<double> o;
 #pragma unroll
-    for (int k = 0; k < kC; ++k) o.v[k] = zz.v[k] + beta.v[k] * pp.v[k];
+    for (int k = 0; k < kC; ++k) o.v[k] = fma(beta.v[k], pp.v[k], zz.v[k]);
     return o;
   }
 };
@@ -513,8 +513,9 @@ struct Tpg {
 
 // ---------------------------------------------------------------------------------------
 // batched V-cycle kernels (same arithmetic per case as the single-RHS smoother kernels);
-// vectors of type T use the case map of T.  The epilogues' products and sums are written as
-// explicit fma: left to the compiler, the 8-wide build contracted them otherwise than the others.
+// vectors of type T use the case map of T.  Products that are added are written as explicit fma here
+// and in all kernels of this file: left to the compiler, the 8-wide build contracted some otherwise
+// than the others, and a case's bits must not depend on the batch width.
 // ---------------------------------------------------------------------------------------
 // xf: the first smoothing step's x, dinv b / theta -- BD0 on the fly, or BLoad of the vector the
 // PCG update wrote (the same values)
@@ -602,7 +603,7 @@ __global__ void __launch_bounds__(kThreads, (kRowCtas<T, BS * BS>))
         if (part) {
           const C4<T> bv = ldc<T>(b + o, l);
 #pragma unroll
-          for (int k = 0; k < kC; ++k) dot[k] += (double)bv.v[k] * (double)xn.v[k];
+          for (int k = 0; k < kC; ++k) dot[k] = fma((double)bv.v[k], (double)xn.v[k], dot[k]);
         }
       }
     }
@@ -666,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, (kRowCtas<T, BS * BS>))
           ro.v[k] = di * (bv.v[k] - acc[rr][k]);
           dd.v[k] = ro.v[k] * inv_theta;
           xn.v[k] = fma(ro.v[k], inv_theta, xv.v[k]);
-          if (part) dot[k] += (double)bv.v[k] * (double)xn.v[k];
+          if (part) dot[k] = fma((double)bv.v[k], (double)xn.v[k], dot[k]);
         }
         if (r) {  // a Chebyshev step follows
           stc<T>(r + o, l, ro);
@@ -863,7 +864,7 @@ struct BEpiCheb {  // r -= D^-1 A d_in; d_out = c1 d_in + c2 r; x += d_out; dot:
     if (want_dot) {
       const C4<T> bv = ldc<T>(b + o, l);
 #pragma unroll
-      for (int k = 0; k < kC; ++k) dot[k] += (double)bv.v[k] * (double)xn.v[k];
+      for (int k = 0; k < kC; ++k) dot[k] = fma((double)bv.v[k], (double)xn.v[k], dot[k]);
     }
   }
 };
@@ -901,7 +902,7 @@ struct BEpiPostFirst {  // r0 = D^-1 (b - A x), d0 = r0 / theta, x2 = x + d0; do
       ro.v[k] = di * (bv.v[k] - acc[k]);
       dd.v[k] = ro.v[k] * inv_theta;
       xn.v[k] = fma(ro.v[k], inv_theta, xv.v[k]);
-      if (want_dot) dot[k] += (double)bv.v[k] * (double)xn.v[k];
+      if (want_dot) dot[k] = fma((double)bv.v[k], (double)xn.v[k], dot[k]);
     }
     if (r) {  // a Chebyshev step follows
       stc<T>(r + o, l, ro);
@@ -924,7 +925,7 @@ struct BEpiSpmvDot {  // p_new = z + beta p_old; q = A p_new; dot: p_new . q
 #pragma unroll
     for (int k = 0; k < kC; ++k) {
       qv.v[k] = acc[k];
-      dot[k] += pv.v[k] * qv.v[k];
+      dot[k] = fma(pv.v[k], qv.v[k], dot[k]);
     }
     stc<double>(p_new + o, l, pv);
     stc<double>(q + o, l, qv);
@@ -1256,7 +1257,7 @@ __global__ void __launch_bounds__(kThreads) kb_coarse(int64_t n, const double* _
       if (col < n) {
         const double bv = (double)b[col * kBatch + j];
 #pragma unroll
-        for (int r = 0; r < kCoarseRows; ++r) s[u][r] += __ldg(rowp[r] + col) * bv;
+        for (int r = 0; r < kCoarseRows; ++r) s[u][r] = fma(__ldg(rowp[r] + col), bv, s[u][r]);
       }
     }
   }
@@ -1292,7 +1293,7 @@ __global__ void __launch_bounds__(kThreads) kb_init_vecs(int64_t n, const double
       stc<double>(x + o, l, C4<double>{});
       if (rm) stc<double>(rm + o, l, cvt4<TM>(v));
 #pragma unroll
-      for (int k = 0; k < kC; ++k) dot[k] += v.v[k] * v.v[k];
+      for (int k = 0; k < kC; ++k) dot[k] = fma(v.v[k], v.v[k], dot[k]);
     }
   }
   write_case_parts<double>(dot, partC);
@@ -1346,7 +1347,7 @@ __global__ void __launch_bounds__(kThreads) kb_prec_vec(int64_t n, const T* __re
 #pragma unroll
       for (int k = 0; k < kC; ++k) {
         zv.v[k] = jacobi ? di * rv.v[k] : rv.v[k];
-        dot[k] += (double)rv.v[k] * (double)zv.v[k];
+        dot[k] = fma((double)rv.v[k], (double)zv.v[k], dot[k]);
       }
       stc<T>(z + o, l, zv);
     }
@@ -1412,7 +1413,7 @@ __global__ void __launch_bounds__(kThreads, (kRowCtas<double, 9>))
 #pragma unroll
         for (int k = 0; k < kC; ++k) {
           qv.v[k] = acc[rr][k];
-          dot[k] += pv.v[k] * qv.v[k];
+          dot[k] = fma(pv.v[k], qv.v[k], dot[k]);
         }
         stc<double>(p_new + o, l, pv);
         stc<double>(q + o, l, qv);
@@ -1440,7 +1441,7 @@ __global__ void __launch_bounds__(kThreads) kb_pnew32(int64_t n, const TM* __res
     const C4<float> pp = ldc<float>(p + o, l);
     C4<float> pn;
 #pragma unroll
-    for (int k = 0; k < kC; ++k) pn.v[k] = (float)(zz.v[k] + b.v[k] * (double)pp.v[k]);
+    for (int k = 0; k < kC; ++k) pn.v[k] = (float)fma(b.v[k], (double)pp.v[k], zz.v[k]);
     stc<float>(p + o, l, pn);
   }
 }
@@ -1472,7 +1473,7 @@ __global__ void __launch_bounds__(kThreads, (kRowCtas<double, 9>))
 #pragma unroll
         for (int k = 0; k < kC; ++k) {
           qv.v[k] = acc[rr][k];
-          dot[k] += pv.v[k] * qv.v[k];
+          dot[k] = fma(pv.v[k], qv.v[k], dot[k]);
         }
         stc<float>(q + i * kBatch, l, qv);
       }
@@ -1520,10 +1521,10 @@ __global__ void __launch_bounds__(kThreads) kb_update(int64_t n, double* __restr
 #pragma unroll
       for (int k = 0; k < kC; ++k) {
         if (a.v[k] != 0.0) {  // finished cases keep x and r exactly (their p may be anything)
-          xv.v[k] += a.v[k] * pv.v[k];
-          rv.v[k] -= a.v[k] * qv.v[k];
+          xv.v[k] = fma(a.v[k], pv.v[k], xv.v[k]);
+          rv.v[k] = fma(-a.v[k], qv.v[k], rv.v[k]);
         }
-        dot[k] += rv.v[k] * rv.v[k];
+        dot[k] = fma(rv.v[k], rv.v[k], dot[k]);
       }
       stc<double>(x + o, l, xv);
       stc<double>(r + o, l, rv);
@@ -1614,7 +1615,7 @@ struct DdAcc {
       two_prod(a, x.hi.v[k], p, ep);
       two_sum(s[r][k], p, t, es);
       s[r][k] = t;
-      c[r][k] += (ep + es) + a * x.lo.v[k];
+      c[r][k] += fma(a, x.lo.v[k], ep + es);
     }
   }
 };
@@ -1645,7 +1646,7 @@ __global__ void __launch_bounds__(kThreads, (kRowCtas<double, 9>))
           double t, e;
           two_sum(fv.v[k], -s[rr][k], t, e);
           rv.v[k] = t + (e - c[rr][k]);
-          dot[k] += rv.v[k] * rv.v[k];
+          dot[k] = fma(rv.v[k], rv.v[k], dot[k]);
         }
         stc<double>(R + o, l, rv);
       }
@@ -1677,7 +1678,7 @@ __global__ void __launch_bounds__(kThreads) kb_dot_pair(int64_t n, const T* __re
     BATCH_DOF_LOOP(n) {
       const C4<T> av = ldc<T>(a + i * kBatch, l), bv = ldc<T>(b + i * kBatch, l);
 #pragma unroll
-      for (int k = 0; k < kC; ++k) dot[k] += (double)av.v[k] * (double)bv.v[k];
+      for (int k = 0; k < kC; ++k) dot[k] = fma((double)av.v[k], (double)bv.v[k], dot[k]);
     }
   }
   write_case_parts<T>(dot, part);
@@ -1691,7 +1692,7 @@ __global__ void __launch_bounds__(kThreads) kb_dot_self(int64_t n, const double*
     BATCH_DOF_LOOP(n) {
       const C4<double> v = ldc<double>(x + i * kBatch, l);
 #pragma unroll
-      for (int k = 0; k < kC; ++k) dot[k] += v.v[k] * v.v[k];
+      for (int k = 0; k < kC; ++k) dot[k] = fma(v.v[k], v.v[k], dot[k]);
     }
   }
   write_case_parts<double>(dot, partC);
