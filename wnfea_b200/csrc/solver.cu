@@ -1131,11 +1131,11 @@ static bool launch_stream_rows(const StreamMat& m, XF xf, EPI epi, double* part,
 // ---------------------------------------------------------------------------------------
 // The coarse levels of a solid with little surface have rows of 100 to 500 blocks and few of them
 // (the 162,000-element block: 2,116 rows of 413 blocks, then 385 of 343), and a restriction's rows are
-// as long.  A warp per row walks such a row in up to 16 dependent rounds of 32 blocks while most
-// of the SMs' warps have no row, and a streamed tile of 256 blocks holds one row, which one of its
-// eight consumer warps computes.  Here a row is spread over W warps, a lane takes its blocks W x 32
-// apart, and its first block's values and column -- which no kernel of the solve writes -- are
-// loaded before griddepcontrol.wait, while the previous kernel finishes.
+// as long.  No streamed tile holds a row of over 256 blocks (6x3: 512), and a warp per row walks such a
+// row in up to 16 dependent rounds of 32 blocks while most of the SMs' warps have no row.  Here a row is
+// spread over W warps, a lane takes its blocks W x 32 apart, and its first block's values and
+// column -- which no kernel of the solve writes -- are loaded before griddepcontrol.wait, while
+// the previous kernel finishes.
 
 template <int BC, int W, typename T, typename XF, typename EPI>
 __global__ void __launch_bounds__(kThreads) k_team_rows(int64_t n_rows, const int32_t* __restrict__ rp,
@@ -1202,26 +1202,27 @@ __global__ void __launch_bounds__(kThreads) k_team_rows(int64_t n_rows, const in
   if (part) write_part(dot, part, sh);
 }
 
-// Warps per row for a matrix of 6-row blocks by its mean blocks per row, 0: the streamed or
-// warp-per-row kernels.  Measured (FP32, event-timed, warp-per-row or streamed -> teams):
-//   no pack: 413 blocks, 130 MB  43 -> 33 us; 343, 20 MB  21 -> 12 us; restrictions of 27 / 2.5 MB
-//            45 -> 14 and 26 -> 10 us;
-//   packed:  243, 76 MB  38 -> 24 us; but 134, 300 MB  76 -> 78 us, 105 (6x3), 140 MB  33 -> 42 us, and
-//            100, 30 MB  10.4 -> 11.8 us on the I-beam's level 2 (its solve 31.9 -> 33.1 ms: the streamed
-//            kernels before and after it lose their overlap too): a pack streams better until a row
-//            fills most of a tile.
-static int team_width(int64_t n_rows, int64_t nnzb, bool packed) {
+// Warps per row for a matrix of 6-row blocks without a pack (under wn_amg_params.stream_min_mb, or with a row
+// that no tile holds) by its mean blocks per row, 0: the warp-per-row kernels.  Measured (FP32,
+// event-timed, warp per row -> teams): 413 blocks, 130 MB  43 -> 33 us; 343, 20 MB  21 -> 12 us;
+// restrictions of 243 blocks, 76 MB  38 -> 24 us, and of 27 / 2.5 MB  45 -> 14 and 26 -> 10 us.
+// A matrix with a pack is streamed whatever its rows: with tiles of few rows shared by the consumer warps
+// that is faster than teams on every matrix of 20 MB and more between 63 and 212 blocks per row, in both
+// precisions (teams -> streamed, FP32 / FP64: 70 blocks, 120 MB in FP32  36 -> 29 / 62 -> 48 us; 134,
+// 290 MB  67 -> 58 / 131 -> 108; 173 (6x3), 83 MB  29 -> 25 / 46 -> 39; 212 (6x3), 69 MB  25 -> 22 /
+// 42 -> 35), and within 0.5 us of them on smaller ones; only one of 256 rows of 251 blocks, 9 MB, is
+// slower (8.2 -> 8.5 / 10.3 -> 11.9).
+static int team_width(int64_t n_rows, int64_t nnzb) {
   if (n_rows <= 0) return 0;
   const double avg = (double)nnzb / (double)n_rows;
-  if (avg < (packed ? 192.0 : 64.0)) return 0;
-  return avg >= 160.0 ? 8 : 4;
+  return avg >= 160.0 ? 8 : avg >= 64.0 ? 4 : 0;
 }
 
 template <int BC, typename T, typename XF, typename EPI>
 static bool launch_team_rows(int64_t n_rows, int64_t nnzb, bool packed, const int32_t* rp, const int32_t* ci,
                              const T* av, XF xf, EPI epi, double* part, const PcgScalars* S, cudaStream_t st,
                              int* grid_out) {
-  const int w = team_width(n_rows, nnzb, packed);
+  const int w = packed ? 0 : team_width(n_rows, nnzb);
   if (w == 0) return false;
   auto go = [&](auto kern, int rows_per_cta) {
     const int g = resident_grid(kern, kThreads, (n_rows + rows_per_cta - 1) / rows_per_cta);
@@ -1233,7 +1234,7 @@ static bool launch_team_rows(int64_t n_rows, int64_t nnzb, bool packed, const in
   return ok;
 }
 
-// y = M x or y += M x for a transfer operator: long rows by teams of warps, else streamed from its
+// y = M x or y += M x for a transfer operator: long rows without a pack by teams of warps, else streamed from its
 // pack when it has one, else the register row kernel
 // (SC: (M x)_i scaled by ys_i -- the FP16 V-cycle's prolongation into its scaled fine level)
 template <int BR, int BC, typename T, bool SC = false>
