@@ -125,8 +125,8 @@ int wn_spmv_solid_device(void* h, int precision, const void* x, void* y, uintptr
 int wn_solid_set_stream(void* h, int enable);
 /* Batched solves (wn_solve_multi*): the FP32 fine-level passes with each row tile's x slice
  * (the 32 cases of the tile's column nodes) staged in shared memory (enable != 0), or the
- * register row kernels gathering x through L1/L2 (0, the default: on the 1M-DOF I-beam the
- * staged passes are slower: 312 ms per 32-case batch).  The same arithmetic in the same
+ * register row kernels gathering x through L1/L2 (0, the default: 154 ms per 32-case batch on
+ * the 1M-DOF I-beam, where the staged passes took 312 ms).  The same arithmetic in the same
  * order: the row products are bitwise the same.  Synchronises. */
 int wn_solid_set_batch_staging(void* h, int enable);
 /* Status word of the streamed fine-matrix products of wn_spmv_solid_device: WN_OK, or
@@ -245,8 +245,11 @@ typedef struct wn_solve_params {
   int chunk;          /* iterations per CUDA-graph replay / host convergence check    */
   int use_graph;      /* 1 = replay captured chunks as a CUDA graph                   */
   int profile;        /* 1 = time every kernel of this solve with CUDA events (graphs
-                         off; read back with wn_solve_profile; small systems run
-                         the same kernels one by one); 0 = normal */
+                         off; read back with wn_solve_profile); 0 = normal.  Systems
+                         of at most 2,048 nodes, whose normal solves run in one
+                         kernel, are profiled on the kernels that larger ones use:
+                         in more time, and the same solution (to rounding; bit for
+                         bit in FP64 without AMG on the streamed fine matrix) */
 } wn_solve_params;
 
 typedef struct wn_solve_stats {

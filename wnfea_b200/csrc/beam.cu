@@ -234,7 +234,7 @@ __global__ void beam_dense_kernel(int64_t n_nodes, const int32_t* __restrict__ r
 // return).  Every loop is bounded by n.
 //
 // What bounds it: the serial chain of pivots.  A panel's rows stay in the registers of one CTA
-// (RPT rows of NB columns per thread), so a column costs two barriers, two three-step warp
+// (RPT rows of NB columns per thread), so a column costs one barrier, two three-step warp
 // reductions, a division and its multiply-adds instead of several passes over global memory;
 // NB x RPT is chosen so that the rows that the band leaves fit (dense_lu).  Measured on the
 // 10 x 10 frame (600 DOFs, kb = 65) against the same algorithm over all n rows and columns from

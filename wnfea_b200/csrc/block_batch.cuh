@@ -685,10 +685,10 @@ __global__ void __launch_bounds__(kThreads, (kRowCtas<T, BS * BS>))
 // shared-memory stage ring of stream.cuh (stream_pipeline).  Per tile, a group of 8 lanes per
 // block row (4 rows per warp), lane l owning 4 of the 32 cases; the group walks its row's
 // blocks in order, two blocks' x gathers in flight, and reads each block's 9 values from the
-// stage (the 8 lanes of a group read the same word: a shared-memory broadcast, where the
-// register kernels above load the values coalesced and pass them round with shuffles).  The
-// per-case arithmetic and the order of every multiply-add are those of the register kernels,
-// so both paths give the same bits.
+// stage (the 8 lanes of a group read the same word: a shared-memory broadcast, as the register
+// kernels above read the stages that they fill themselves).  The per-case arithmetic and the order
+// of every multiply-add are those of the register kernels, so both paths give the same bits.  For
+// 32 cases only, and only when switched on (wn_solid_set_stream).
 // ---------------------------------------------------------------------------------------
 // the fine matrix in one precision as the streamed kernels see it
 struct BView {
@@ -977,16 +977,16 @@ int launch_bs(K kern, const StreamMat& m, cudaStream_t st, Args... args) {
 }
 
 // ---------------------------------------------------------------------------------------
-// fine level with each tile's x slice staged in shared memory (the default for the batched
-// fine level).  An x-tile is a run of whole block rows whose blocks name at most kXTileCols
+// fine level with each tile's x slice staged in shared memory (32 cases, switched on by
+// wn_solid_set_batch_staging).  An x-tile is a run of whole block rows whose blocks name at most kXTileCols
 // distinct column nodes (the plan in BlockWork: per tile the sorted column list, per block its
 // column as an 8-bit index into that list).  The CTA first writes the x values of the tile's
 // columns -- xf(i, l) for the 32 cases of each of their DOFs, the same functor and arithmetic
 // as the register kernels' gathers -- into shared memory with coalesced 16-byte loads, many in
-// flight at once; then 8-lane groups run the rows exactly as batch_row_staged does (stages of 8
-// blocks, values component-major and coalesced, broadcast by shuffles; the same order of every
-// multiply-add, so the same bits) but read each block's x from shared memory by its local
-// column.  A gathered x row served 2-3 blocks of the tile from L1/L2 before (the tiles' column
+// flight at once; then 8-lane groups run the rows in stages of 8 blocks, values component-major and
+// coalesced, passed round by shuffles (batch_row_staged hands them over in shared memory; the
+// order of every multiply-add is the same, so the bits are too), and read each block's x from shared
+// memory by its local column.  A gathered x row served 2-3 blocks of the tile from L1/L2 before (the tiles' column
 // lists hold 2.8 M rows against 8.5 M blocks on the I-beam), and the gathers' latency was what
 // bound the batched sweeps.
 // ---------------------------------------------------------------------------------------

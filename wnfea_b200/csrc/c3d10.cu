@@ -27,12 +27,13 @@ __constant__ unsigned char c_tri_b[55] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 1, 2, 3,
 constexpr int KE_TILE = 16;      // elements per CTA
 constexpr int KE_THREADS = 256;  // threads per CTA
 
-// Stage one element's coordinates: X[a][j] = nodes[conn[e][a]][j].
+// an asynchronous 4-byte copy to shared memory
 __device__ __forceinline__ void cp_async4(int32_t* smem, const int32_t* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(gmem) : "memory");
 }
 
+// Stage one element's coordinates: X[a][j] = nodes[conn[e][a]][j].
 __device__ __forceinline__ void load_coords(const double* __restrict__ nodes, const int32_t* __restrict__ conn,
                                             int64_t e, double X[10][3]) {
 #pragma unroll

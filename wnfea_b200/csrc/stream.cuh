@@ -381,8 +381,8 @@ struct NoHook {
 // Cfg's capacities (NV = BR * BC values per block).  The producer warp streams the CTA's run of
 // tiles into the stage ring; every consumer warp calls body(jc, stage, desc, dot) for each tile jc
 // of the run (stage = the tile's image in shared memory, desc = rows r0, r1 / segment /
-// cntp; false: a bounded wait of the body ran out), adding its dot contributions to the consumer's running sum, which is returned (0 for
-// the producer).
+// cntp; false: a bounded wait of the body ran out), adding its dot contributions to the consumer's
+// running sum, which is returned (0 for the producer).
 // The first stages' copies (the matrix only) are issued before pdl_wait(), so under a
 // programmatic dependent launch they overlap the predecessor's tail; then every thread runs
 // hook(), and when *done is set (read after the wait) the CTA lets those copies land and
