@@ -4,6 +4,8 @@ the solve stops at its iteration limit, and no solve runs twice."""
 
 from __future__ import annotations
 
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -83,3 +85,26 @@ def test_long_amg_solve_takes_several_launches(cells, precision):
     # the launched kernels' sums run in another order; a lost direction would cost a start from scratch
     assert abs(st["iterations"] - sv["iterations"]) <= 0.05 * sv["iterations"]
     assert np.linalg.norm(u - v) <= 1e-9 * np.linalg.norm(v)
+
+
+# tetrahedra apart from one another, clamped on a face: rows of 10 blocks, so that a row tile has 51 rows and a warp's
+# share of it two passes
+@pytest.mark.parametrize("precond", [0, 1, 3])
+def test_tiles_of_many_short_rows(precond):
+    m, _ = generate_c3d10_kuhn_block(1.0, 1.0, 1.0, 1, 1, 1)
+    tet = m.mesh_nodes[m.solid_elements[0]]
+    rng = np.random.default_rng(5)
+    n_tets = 57
+    scale = rng.uniform(0.2, 3.0, (n_tets, 1, 1))
+    nodes = (scale * tet + 4.0 * np.arange(n_tets)[:, None, None]).reshape(-1, 3)
+    face = [0, 1, 2, 4, 5, 6]  # vertices 0, 1, 2 and the nodes amid their edges
+    supports = [dataclasses.replace(m.supports[0], node_id=10 * t + a) for t in range(n_tets) for a in face]
+    m = dataclasses.replace(m, mesh_nodes=nodes, solid_elements=np.arange(10 * n_tets, dtype=np.int32).reshape(-1, 10),
+                            supports=supports, loads=[])
+    K, _, _ = assemble_c3d10_sparse_3dof(m)
+    s = K.system
+    assert np.all(np.diff(s.pattern()[0]) == 10)
+    F = rng.standard_normal(K.shape[0]) * 100.0
+    F[np.asarray(solid_fixed_dofs(m), dtype=np.int64)] = 0.0
+    st = _same(s, F, rtol=1e-10, max_iter=2000, precond=precond)
+    assert st["iterations"] > 3 and (precond == 0 or st["status"] == 0)
